@@ -66,6 +66,14 @@ struct co_bufs {
     float4 *pf_x;        // {x1h, x2h, x1l, x2l}
     float4 *pf_g;        // {g1h, g2h, g1l, g2l}
     float *pf_w, *pf_wl; // weight head / tail
+    // fixed-point operands of the FP64-accurate pair sum (co_pair_fixed.cu): X1, X2
+    // per marker, G in limbs, the scaled weights (also as FP64),
+    // the scales {into, out of} the scaled units, and the pack kernel's block
+    // maxima (|G|, |w|)
+    long long *fx_x, *fx_w;
+    int4 *fx_g;
+    double *pwn, *unit;
+    double2 *gwmax;
     double *pdot;        // packed vdot (2 x cap)
     double *pA;          // packed metric A (3 x cap)
     double *part;        // slice partials of the pair kernels
@@ -145,6 +153,7 @@ struct co_ctx {
     int pair_split_fp64, pair_split_fp32;  // split factors of the plain kernels (0 = auto)
     int pair_symmetric;      // 1: Newton's-third-law kernels (default), 0: one-sided
     int nsm;
+    int fixed_ex;            // exponent of the fixed-point pair sum's coordinate scale
     // launch counter (kernels of this library launched through the context)
     unsigned long long launches;
     // pair-kernel profiling (co_prof.cu)
@@ -210,9 +219,8 @@ int co_features_res_dev(co_ctx *c, int N, const double *r, double dt, float *X);
 // (co_pair.cu)
 int co_pair_fp64(co_ctx *c, int M, int with_metric);   // packed -> pdot (and pA)
 int co_pair_fp32(co_ctx *c, int M);                    // packed FP32 -> pdot
-int co_pair_ds(co_ctx *c, int M);                      // packed FP32 head/tail -> pdot,
-                                                       // double-single arithmetic
-int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez);
+int co_pair_ds(co_ctx *c, int M);                      // packed -> pdot, double-single form
+int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez, int batch = 0);
 int co_pack_plain(co_ctx *c, int N, int Mub, int precision, const double *x, const double *G);
 int co_unpack_A(co_ctx *c, int N, double *A);
 int co_metric32(co_ctx *c, int Mub);   // FP32 metric A (3 x ld in pA) from pf_x/pf_w
@@ -227,10 +235,32 @@ int co_step_newton_buffers(co_ctx *c, const co_opts *o, const co_newton_opts *nk
                            double S0, double dt, int *evals, double *res, int *n_newton,
                            double *r0, int *status);
 #define CO_PREC_BOTH 3                  // pack both FP64 and FP32 operands (internal)
-// packed-operand sets a precision needs: 1 = FP64 arrays, 2 = FP32 head/tail arrays
+// packed-operand sets a precision needs: 1 = FP64 arrays (from which the
+// fixed-point operands are made), 2 = FP32 head/tail arrays; a double-single sum below
+// the symmetric kernel's smallest size takes the FP64 ones
 static inline int co_pack_mode(int precision) {
-    return precision == CO_PREC_FP64 ? 1 : precision == CO_PREC_BOTH ? 3 : 2;
+    return precision == CO_PREC_FP64 ? 1 : precision == CO_PREC_MIXED ? 2 : 3;
 }
+// Whether an FP64-accurate pair sum of up to Mub markers takes the fixed-point
+// kernel: from four 128-marker tiles on; below that the one-sided FP64 kernel's
+// single launch is as fast. The one-sided FP64 form also stays for CO_FLAG_ONESIDED.
+static inline int co_use_fixed(const co_ctx *c, int Mub, int precision) {
+    return (precision == CO_PREC_FP64 || precision == CO_PREC_BOTH) && c->pair_symmetric &&
+           co_cdiv(Mub, 128) >= 4;
+}
+// operands of the fixed-point pair sum, as the kernels take them
+struct co_fixed_ops {
+    const longlong2 *x;     // coordinates
+    const int4 *g;          // gradients: two limbs per component
+    const long long *w;     // weights
+    const double2 *px, *pg; // FP64 operands (close pairs)
+    const double *pwn, *unit;
+    float m_close;          // a pair whose larger |d| component is below takes the FP64 form
+};
+int co_pair_fixed_pack(co_ctx *c, int Mub, int npart);  // px, pg, pw -> fixed-point operands
+int co_pair_fixed_sum(co_ctx *c, int Mub, int metric, int prof_kind);  // -> pdot (and pA)
+co_fixed_ops co_fixed_operands(co_ctx *c);
+int co_ensure_part(co_ctx *c, size_t n);
 int co_unpack_update(co_ctx *c, int N, double dt, double *Gv, const double *v0,
                      const double *v1, double *r, double *red);
 

@@ -7,9 +7,11 @@
 // into slices whose partial sums are added afterwards in slice order, so
 // results are bitwise reproducible for a given N.
 //
-// FP64 form (the reference's Float64 path): on GB300 FP64 issues at 1/64 of
-// the FP32 rate, so the per-pair FP64 instruction count is what sets the time.
-// The pair body is 20 FP64 instructions:
+// The reference's Float64 path runs on the fixed-point kernels of co_pair_fixed.cu;
+// the FP64 arithmetic below serves the one-sided kernels (CO_FLAG_ONESIDED, fewer
+// than 385 markers) and the batched one. On GB300 FP64 issues at 1/64 of the FP32
+// rate, so the per-pair FP64 instruction count is what sets its time. The pair body
+// is 20 FP64 instructions:
 //   d (2), |d|^2 (2), 1/|d| refinement (5), G difference (2), d.g (2),
 //   1/|d|^2 and (d.g)/|d|^2 (2), projection (2), w/|d| (1), accumulate (2).
 // 1/|d| starts from a single-precision seed built from the FP64 bit pattern
@@ -344,69 +346,6 @@ __device__ __forceinline__ bool sym_skip(int nt, int H, int I, int k) {
     return k > 0 && (nt & 1) == 0 && k == H && I >= nt / 2;
 }
 
-__global__ void __launch_bounds__(ST)
-k_pair64_sym(const double2 *__restrict__ px, const double2 *__restrict__ pg,
-             const double *__restrict__ pw, int nt, int H, int KC,
-             double *__restrict__ gpart, double *__restrict__ apart) {
-    __shared__ double2 sx[ST], sg[ST];
-    __shared__ double sw[ST];
-    __shared__ double2 sacc[ST];
-    const int I = blockIdx.x % nt, chunk = blockIdx.x / nt;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const double2 xg = px[I * ST + tid], Gg = pg[I * ST + tid];
-    const double wg = pw[I * ST + tid];
-    double ga1 = 0.0, ga2 = 0.0;
-    const int k0 = chunk * KC, k1 = min(H + 1, k0 + KC);
-    for (int k = k0; k < k1; k++) {
-        if (sym_skip(nt, H, I, k)) continue;
-        const int J = (I + k) % nt;
-        __syncthreads();
-        sx[tid] = px[J * ST + tid];
-        sg[tid] = pg[J * ST + tid];
-        sw[tid] = pw[J * ST + tid];
-        sacc[tid] = make_double2(0.0, 0.0);
-        __syncthreads();
-        if (k == 0) {  // diagonal tile: ordered pairs, self excluded by the guard
-#pragma unroll 4
-            for (int a = 0; a < ST; a++) {
-                double u1, u2;
-                double2 xa = sx[a], Ga = sg[a];
-                pair_u64(xg.x - xa.x, xg.y - xa.y, Ga.x - Gg.x, Ga.y - Gg.y, u1, u2);
-                ga1 = fma(sw[a], u1, ga1);
-                ga2 = fma(sw[a], u2, ga2);
-            }
-            continue;
-        }
-        for (int r = 0; r < 4; r++) {
-            const int base = ((warp + r) & 3) * 32;
-            double2 a0 = sacc[base + lane];
-            double a1 = a0.x, a2 = a0.y;
-#pragma unroll 4
-            for (int q = 0; q < 32; q++) {
-                const int ai = base + ((lane + q) & 31);
-                double2 xa = sx[ai], Ga = sg[ai];
-                double wa = sw[ai];
-                double u1, u2;
-                pair_u64(xg.x - xa.x, xg.y - xa.y, Ga.x - Gg.x, Ga.y - Gg.y, u1, u2);
-                ga1 = fma(wa, u1, ga1);
-                ga2 = fma(wa, u2, ga2);
-                a1 = fma(-wg, u1, a1);
-                a2 = fma(-wg, u2, a2);
-                a1 = __shfl_sync(0xffffffffu, a1, (lane + 1) & 31);
-                a2 = __shfl_sync(0xffffffffu, a2, (lane + 1) & 31);
-            }
-            sacc[base + lane] = make_double2(a1, a2);
-            __syncthreads();
-        }
-        double *ap = apart + ((size_t)(k - 1) * nt + J) * 2 * ST;
-        ap[tid] = sacc[tid].x;
-        ap[ST + tid] = sacc[tid].y;
-    }
-    double *gp = gpart + ((size_t)chunk * nt + I) * 2 * ST;
-    gp[tid] = ga1;
-    gp[ST + tid] = ga2;
-}
-
 // FP32 body on head/tail operands: returns the unweighted term u
 __device__ __forceinline__ void pair_u32(const float4 &xg, const float4 &Gg, const float4 &xa,
                                          const float4 &Ga, float &u1, float &u2) {
@@ -544,7 +483,7 @@ k_pair32_sym(const float4 *__restrict__ pfx, const float4 *__restrict__ pfg,
 // __fadd_rn/__fsub_rn/__fmul_rn/__fmaf_rn keep the compiler from contracting
 // these sequences. 1/|d| is one Newton step from the MUFU seed. Each unordered
 // pair (both orders) costs about 190 FP32 instructions against 20 FP64
-// instructions in k_pair64_sym, i.e. about 7x less issue time on a part whose
+// instructions of the FP64 form, i.e. about 7x less issue time on a part whose
 // FP32:FP64 rate is 64:1, at ~1e-13 relative accuracy per term; momentum stays
 // exact to the accumulation round-off because each pair's term is computed once
 // and added with both signs. Used for the FP64 stage of the mixed precision form.
@@ -927,92 +866,99 @@ __global__ void k_slice_reduce(const double *__restrict__ part, int split, int n
     }
 }
 
-// Landau pack: lambda from the device state, G_eff = -(dS + lambda dv)/w
-// (solver.jl:107-111), operands in sorted order.
-__global__ void k_pack_landau(const int *__restrict__ perm, const int *__restrict__ Mp, int Mpad, int N,
-                              const double *__restrict__ vmid, const double *__restrict__ dS,
-                              const double *__restrict__ dv, const double *__restrict__ w,
-                              const co_solver_state *__restrict__ st, int use_lambda,
-                              int mode, double2 *__restrict__ px, double2 *__restrict__ pg,
-                              double *__restrict__ pw, float4 *__restrict__ pfx,
-                              float4 *__restrict__ pfg, float *__restrict__ pfw, float *__restrict__ pfwl) {
-    int M = *Mp;
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= Mpad) return;
-    if (p >= M) {  // inert padding up to the tile boundary: far away, zero weight
-        if (mode & 2) {
-            pfx[p] = make_float4(1e3f, 1e3f, 0.f, 0.f);
-            pfg[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-            pfw[p] = 0.f;
-            pfwl[p] = 0.f;
-        }
-        if (mode & 1) {
-            px[p] = make_double2(1e3, 1e3);
-            pg[p] = make_double2(0.0, 0.0);
-            pw[p] = 0.0;
-        }
-        return;
-    }
-    int a = perm[p];
-    double lam = use_lambda ? st->lambda : 0.0;
-    double iw = 1.0 / w[a];
-    double x1 = vmid[a], x2 = vmid[N + a];
-    double G1 = -(dS[a] + lam * dv[a]) * iw;
-    double G2 = -(dS[N + a] + lam * dv[N + a]) * iw;
+// Packed operands of one sorted position, by mode bit: 1 FP64, 2 FP32 head/tail.
+// Positions M .. Mpad are inert padding up to the tile boundary: far away, zero
+// weight.
+struct co_pack_out {
+    double2 *px, *pg;
+    double *pw;
+    float4 *pfx, *pfg;
+    float *pfw, *pfwl;
+    double2 *gwmax;   // block maxima of |G| and |w| (the fixed-point scales)
+};
+
+__device__ __forceinline__ void pack_store(const co_pack_out &o, int mode, int p, bool in,
+                                           double x1, double x2, double G1, double G2, double w) {
     if (mode & 2) {
-        float x1h = (float)x1, x2h = (float)x2, G1h = (float)G1, G2h = (float)G2;
-        pfx[p] = make_float4(x1h, x2h, (float)(x1 - (double)x1h), (float)(x2 - (double)x2h));
-        pfg[p] = make_float4(G1h, G2h, (float)(G1 - (double)G1h), (float)(G2 - (double)G2h));
-        float wh = (float)w[a];
-        pfw[p] = wh;
-        pfwl[p] = (float)(w[a] - (double)wh);
+        const float x1h = in ? (float)x1 : 1e3f, x2h = in ? (float)x2 : 1e3f;
+        const float G1h = (float)G1, G2h = (float)G2;
+        o.pfx[p] = make_float4(x1h, x2h, in ? (float)(x1 - (double)x1h) : 0.f,
+                               in ? (float)(x2 - (double)x2h) : 0.f);
+        o.pfg[p] = make_float4(G1h, G2h, (float)(G1 - (double)G1h), (float)(G2 - (double)G2h));
+        const float wh = (float)w;
+        o.pfw[p] = wh;
+        o.pfwl[p] = (float)(w - (double)wh);
     }
     if (mode & 1) {
-        px[p] = make_double2(x1, x2);
-        pg[p] = make_double2(G1, G2);
-        pw[p] = w[a];
+        o.px[p] = in ? make_double2(x1, x2) : make_double2(1e3, 1e3);
+        o.pg[p] = make_double2(G1, G2);
+        o.pw[p] = w;
     }
 }
 
+// block maxima of |G| and |w|; inf where an operand is not finite
+__device__ __forceinline__ void pack_max(const co_pack_out &o, double x1, double x2, double G1,
+                                         double G2, double w) {
+    __shared__ double2 sh[8];
+    double gm = fmax(fabs(G1), fabs(G2)), wm = fabs(w);
+    if (!isfinite(x1 + x2) || !isfinite(G1) || !isfinite(G2) || !isfinite(w)) gm = INFINITY;
+    for (int s = 16; s > 0; s >>= 1) {
+        gm = fmax(gm, __shfl_xor_sync(0xffffffffu, gm, s));
+        wm = fmax(wm, __shfl_xor_sync(0xffffffffu, wm, s));
+    }
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = make_double2(gm, wm);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < (int)(blockDim.x >> 5); i++) {
+            gm = fmax(gm, sh[i].x);
+            wm = fmax(wm, sh[i].y);
+        }
+        o.gwmax[blockIdx.x] = make_double2(gm, wm);
+    }
+}
+
+// Landau pack: lambda from the device state, G_eff = -(dS + lambda dv)/w
+// (solver.jl:107-111), operands in sorted order.
+__global__ void __launch_bounds__(256)
+k_pack_landau(const int *__restrict__ perm, const int *__restrict__ Mp, int Mpad, int N,
+              const double *__restrict__ vmid, const double *__restrict__ dS,
+              const double *__restrict__ dv, const double *__restrict__ w,
+              const co_solver_state *__restrict__ st, int use_lambda, int mode, co_pack_out o) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = p < *Mp;
+    double x1 = 0.0, x2 = 0.0, G1 = 0.0, G2 = 0.0, wa = 0.0;
+    if (in) {
+        const int a = perm[p];
+        const double lam = use_lambda ? st->lambda : 0.0;
+        wa = w[a];
+        const double iw = 1.0 / wa;
+        x1 = vmid[a];
+        x2 = vmid[N + a];
+        G1 = -(dS[a] + lam * dv[a]) * iw;
+        G2 = -(dS[N + a] + lam * dv[N + a]) * iw;
+    }
+    if (p < Mpad) pack_store(o, mode, p, in, x1, x2, G1, G2, wa);
+    if (mode & 1) pack_max(o, x1, x2, G1, G2, wa);
+}
+
 // Hook pack: operands straight from (v, G, w) (COLLISION_FN semantics).
-__global__ void k_pack_plain(const int *__restrict__ perm, const int *__restrict__ Mp, int Mpad, int N,
-                             const double *__restrict__ v, const double *__restrict__ G,
-                             const double *__restrict__ w, int mode,
-                             double2 *__restrict__ px, double2 *__restrict__ pg,
-                             double *__restrict__ pw, float4 *__restrict__ pfx,
-                             float4 *__restrict__ pfg, float *__restrict__ pfw, float *__restrict__ pfwl) {
-    int M = *Mp;
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= Mpad) return;
-    if (p >= M) {  // inert padding up to the tile boundary: far away, zero weight
-        if (mode & 2) {
-            pfx[p] = make_float4(1e3f, 1e3f, 0.f, 0.f);
-            pfg[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-            pfw[p] = 0.f;
-            pfwl[p] = 0.f;
-        }
-        if (mode & 1) {
-            px[p] = make_double2(1e3, 1e3);
-            pg[p] = make_double2(0.0, 0.0);
-            pw[p] = 0.0;
-        }
-        return;
+__global__ void __launch_bounds__(256)
+k_pack_plain(const int *__restrict__ perm, const int *__restrict__ Mp, int Mpad, int N,
+             const double *__restrict__ v, const double *__restrict__ G,
+             const double *__restrict__ w, int mode, co_pack_out o) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = p < *Mp;
+    double x1 = 0.0, x2 = 0.0, G1 = 0.0, G2 = 0.0, wa = 0.0;
+    if (in) {
+        const int a = perm[p];
+        x1 = v[a];
+        x2 = v[N + a];
+        G1 = G[a];
+        G2 = G[N + a];
+        wa = w[a];
     }
-    int a = perm[p];
-    double x1 = v[a], x2 = v[N + a], G1 = G[a], G2 = G[N + a];
-    if (mode & 2) {
-        float x1h = (float)x1, x2h = (float)x2, G1h = (float)G1, G2h = (float)G2;
-        pfx[p] = make_float4(x1h, x2h, (float)(x1 - (double)x1h), (float)(x2 - (double)x2h));
-        pfg[p] = make_float4(G1h, G2h, (float)(G1 - (double)G1h), (float)(G2 - (double)G2h));
-        float wh = (float)w[a];
-        pfw[p] = wh;
-        pfwl[p] = (float)(w[a] - (double)wh);
-    }
-    if (mode & 1) {
-        px[p] = make_double2(x1, x2);
-        pg[p] = make_double2(G1, G2);
-        pw[p] = w[a];
-    }
+    if (p < Mpad) pack_store(o, mode, p, in, x1, x2, G1, G2, wa);
+    if (mode & 1) pack_max(o, x1, x2, G1, G2, wa);
 }
 
 // Gv = v0 + dt * vdot (solver.jl:225), vdot unpacked from sorted order (0 for
@@ -1083,7 +1029,7 @@ static int choose_split(co_ctx *c, int M, int tpb, int force) {
     return want;
 }
 
-static int ensure_part(co_ctx *c, size_t n) {
+int co_ensure_part(co_ctx *c, size_t n) {
     if (n <= c->mb.part_cap) return CO_OK;
     if (c->mb.part) cudaFree(c->mb.part);
     c->mb.part = nullptr;
@@ -1093,11 +1039,9 @@ static int ensure_part(co_ctx *c, size_t n) {
 }
 
 // M is an upper bound (N); the true count sits at cstart[n_el] on the device.
-static int pair_sym(co_ctx *c, int Mub, int fp64);
-
 int co_pair_fp64(co_ctx *c, int Mub, int with_metric) {
     if (Mub <= 0) return CO_OK;
-    if (!with_metric && c->pair_symmetric && co_cdiv(Mub, ST) >= 4) return pair_sym(c, Mub, 1);
+    if (co_use_fixed(c, Mub, CO_PREC_FP64)) return co_pair_fixed_sum(c, Mub, with_metric, 1);
     const int *Mp = c->mb.cstart + c->n_el;
     size_t ld = (size_t)c->mb.cap;
     int split = choose_split(c, Mub, PAIR_TPB, c->pair_split_fp64);
@@ -1108,7 +1052,7 @@ int co_pair_fp64(co_ctx *c, int Mub, int with_metric) {
     dim3 grid(co_cdiv(Mub, PAIR_TPB), split);
     double *dst = c->mb.pdot;
     if (split > 1 || with_metric) {
-        int rc = ensure_part(c, (size_t)split * nc * ld);
+        int rc = co_ensure_part(c, (size_t)split * nc * ld);
         if (rc) return rc;
         dst = c->mb.part;
     }
@@ -1139,55 +1083,24 @@ int co_pair_fp64(co_ctx *c, int Mub, int with_metric) {
 
 #define SYM_KC 8
 
-// symmetric pair sum on the padded operands (Mpad = nt * ST);
-// kind: 0 FP32, 1 FP64, 2 double-single
-static int pair_sym(co_ctx *c, int Mub, int kind) {
-    const int fp64 = kind != 0;  // partials of the source side in double
-    int nt = co_cdiv(Mub, ST);
-    int H = nt / 2;
-    int KC = SYM_KC;
-    int nchunk = co_cdiv(H + 1, KC);
-    size_t gsz = (size_t)nchunk * nt * 2 * ST;               // doubles
-    size_t asz = (size_t)(H > 0 ? H : 1) * nt * 2 * ST;      // doubles (fp64) / floats (fp32)
-    size_t need = gsz + (fp64 ? asz : (asz + 1) / 2);
-    if (!fp64) {   // the FP32 kernel's 256-marker tiles
-        const int nt2 = co_cdiv(Mub, 2 * ST), H2 = nt2 / 2, nchunk2 = co_cdiv(H2 + 1, KC);
-        const size_t g2 = (size_t)nchunk2 * nt2 * 4 * ST;
-        const size_t a2 = (size_t)(H2 > 0 ? H2 : 1) * nt2 * 4 * ST;
-        need = g2 + (a2 + 1) / 2;
-    }
-    int rc = ensure_part(c, need);
+// FP32 symmetric pair sum: two targets per thread on 256-marker tiles (Mpad is a
+// multiple of 256 and the tile count has been checked by the caller)
+static int pair32_sym(co_ctx *c, int Mub) {
+    constexpr int R32 = 2, TS32 = R32 * ST;
+    const int KC = SYM_KC;
+    const int nt = co_cdiv(Mub, TS32), H = nt / 2, nchunk = co_cdiv(H + 1, KC);
+    const size_t gsz = (size_t)nchunk * nt * 2 * TS32;
+    const size_t asz = (size_t)(H > 0 ? H : 1) * nt * 2 * TS32;   // floats
+    int rc = co_ensure_part(c, gsz + (asz + 1) / 2);
     if (rc) return rc;
     double *gpart = c->mb.part;
-    co_prof_begin(c, kind == 1 ? 1 : (kind == 2 ? 2 : 0));
-    if (kind == 2) {
-        double *apart = c->mb.part + gsz;
-        k_pair_ds_sym<<<nt * nchunk, ST, 0, c->stream>>>(c->mb.pf_x, c->mb.pf_g, c->mb.pf_w,
-                                                         c->mb.pf_wl, nt, H, KC, gpart, apart);
-        co_prof_end(c);
-        k_sym_reduce<double><<<co_cdiv((long long)nt * ST, 256), 256, 0, c->stream>>>(
-            gpart, apart, nt, H, nchunk, ST, c->mb.pdot, (size_t)c->mb.cap);
-    } else if (fp64) {
-        double *apart = c->mb.part + gsz;
-        k_pair64_sym<<<nt * nchunk, ST, 0, c->stream>>>(c->mb.px, c->mb.pg, c->mb.pw, nt, H, KC,
-                                                        gpart, apart);
-        co_prof_end(c);
-        k_sym_reduce<double><<<co_cdiv((long long)nt * ST, 256), 256, 0, c->stream>>>(
-            gpart, apart, nt, H, nchunk, ST, c->mb.pdot, (size_t)c->mb.cap);
-    } else {
-        // FP32: two targets per thread on 256-marker tiles (Mpad is a multiple of
-        // 256 and the tile count has been checked by the caller)
-        constexpr int R32 = 2, TS32 = R32 * ST;
-        const int nt2 = co_cdiv(Mub, TS32), H2 = nt2 / 2, nchunk2 = co_cdiv(H2 + 1, KC);
-        const size_t gsz2 = (size_t)nchunk2 * nt2 * 2 * TS32;
-        float *apart = (float *)(c->mb.part + gsz2);
-        k_pair32_sym<R32><<<nt2 * nchunk2, ST, 0, c->stream>>>(c->mb.pf_x, c->mb.pf_g,
-                                                               c->mb.pf_w, nt2, H2, KC,
-                                                               gpart, apart);
-        co_prof_end(c);
-        k_sym_reduce<float><<<co_cdiv((long long)nt2 * TS32, 256), 256, 0, c->stream>>>(
-            gpart, apart, nt2, H2, nchunk2, TS32, c->mb.pdot, (size_t)c->mb.cap);
-    }
+    float *apart = (float *)(c->mb.part + gsz);
+    co_prof_begin(c, 0);
+    k_pair32_sym<R32><<<nt * nchunk, ST, 0, c->stream>>>(c->mb.pf_x, c->mb.pf_g, c->mb.pf_w, nt, H,
+                                                         KC, gpart, apart);
+    co_prof_end(c);
+    k_sym_reduce<float><<<co_cdiv((long long)nt * TS32, 256), 256, 0, c->stream>>>(
+        gpart, apart, nt, H, nchunk, TS32, c->mb.pdot, (size_t)c->mb.cap);
     c->launches += 2;
     CO_CK(cudaGetLastError());
     return CO_OK;
@@ -1195,8 +1108,7 @@ static int pair_sym(co_ctx *c, int Mub, int kind) {
 
 int co_pair_fp32(co_ctx *c, int Mub) {
     if (Mub <= 0) return CO_OK;
-    if (c->pair_symmetric && co_cdiv(Mub, 2 * ST) >= 4) return pair_sym(c, Mub, 0);
-    if (Mub <= 0) return CO_OK;
+    if (c->pair_symmetric && co_cdiv(Mub, 2 * ST) >= 4) return pair32_sym(c, Mub);
     const int *Mp = c->mb.cstart + c->n_el;
     size_t ld = (size_t)c->mb.cap;
     int split = choose_split(c, Mub, PAIR_TPB, c->pair_split_fp32);
@@ -1206,7 +1118,7 @@ int co_pair_fp32(co_ctx *c, int Mub) {
     dim3 grid(co_cdiv(Mub, PAIR_TPB), split);
     double *dst = c->mb.pdot;
     if (split > 1) {
-        int rc = ensure_part(c, (size_t)split * 2 * ld);
+        int rc = co_ensure_part(c, (size_t)split * 2 * ld);
         if (rc) return rc;
         dst = c->mb.part;
     }
@@ -1224,30 +1136,36 @@ int co_pair_fp32(co_ctx *c, int Mub) {
     return CO_OK;
 }
 
+static co_pack_out pack_out(co_ctx *c) {
+    co_bufs &b = c->mb;
+    return {b.px, b.pg, b.pw, b.pf_x, b.pf_g, b.pf_w, b.pf_wl, b.gwmax};
+}
+
 int co_pack_plain(co_ctx *c, int N, int Mub, int precision, const double *x, const double *G) {
     if (Mub <= 0) return CO_OK;
     const int *Mp = c->mb.cstart + c->n_el;
     co_bufs &b = c->mb;
     int Mpad = co_cdiv(Mub, 256) * 256;  // whole tiles of up to 256 markers
-    k_pack_plain<<<co_cdiv(Mpad, 256), 256, 0, c->stream>>>(b.perm, Mp, Mpad, N, x, G, b.w,
-                                                            co_pack_mode(precision), b.px, b.pg,
-                                                            b.pw, b.pf_x, b.pf_g, b.pf_w, b.pf_wl);
+    k_pack_plain<<<Mpad / 256, 256, 0, c->stream>>>(b.perm, Mp, Mpad, N, x, G, b.w,
+                                                    co_pack_mode(precision), pack_out(c));
     c->launches++;
     CO_CK(cudaGetLastError());
-    return CO_OK;
+    return co_use_fixed(c, Mub, precision) ? co_pair_fixed_pack(c, Mub, Mpad / 256) : CO_OK;
 }
 
-int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez) {
+// batch != 0: the operands of the batched FP64 kernel only
+int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez, int batch) {
     if (Mub <= 0) return CO_OK;
     const int *Mp = c->mb.cstart + c->n_el;
     co_bufs &b = c->mb;
     int Mpad = co_cdiv(Mub, 256) * 256;  // whole tiles of up to 256 markers
-    k_pack_landau<<<co_cdiv(Mpad, 256), 256, 0, c->stream>>>(
-        b.perm, Mp, Mpad, N, b.vmid, b.dS, b.dv, b.w, c->st, gonzalez, co_pack_mode(precision),
-        b.px, b.pg, b.pw, b.pf_x, b.pf_g, b.pf_w, b.pf_wl);
+    k_pack_landau<<<Mpad / 256, 256, 0, c->stream>>>(b.perm, Mp, Mpad, N, b.vmid, b.dS, b.dv, b.w,
+                                                     c->st, gonzalez, co_pack_mode(precision),
+                                                     pack_out(c));
     c->launches++;
     CO_CK(cudaGetLastError());
-    return CO_OK;
+    return !batch && co_use_fixed(c, Mub, precision) ? co_pair_fixed_pack(c, Mub, Mpad / 256)
+                                                     : CO_OK;
 }
 
 int co_unpack_update(co_ctx *c, int N, double dt, double *Gv, const double *v0,
@@ -1278,7 +1196,7 @@ int co_metric32(co_ctx *c, int Mub) {
         int nt = co_cdiv(Mub, ST), H = nt / 2, KC = SYM_KC, nchunk = co_cdiv(H + 1, KC);
         size_t gsz = (size_t)nchunk * nt * 3 * ST;
         size_t asz = (size_t)(H > 0 ? H : 1) * nt * 3 * ST;  // floats
-        int rc = ensure_part(c, gsz + (asz + 1) / 2);
+        int rc = co_ensure_part(c, gsz + (asz + 1) / 2);
         if (rc) return rc;
         float *apart = (float *)(c->mb.part + gsz);
         k_metric32_sym<<<nt * nchunk, ST, 0, c->stream>>>(c->mb.pf_x, c->mb.pf_w, nt, H, KC,
@@ -1297,18 +1215,31 @@ int co_metric32(co_ctx *c, int Mub) {
     return CO_OK;
 }
 
-// FP64-equivalent pair sum in double-single arithmetic (symmetric kernel);
-// falls back to the FP64 kernel below 4 tiles
+// FP64-equivalent pair sum in double-single arithmetic (symmetric kernel); falls
+// back to the FP64 kernel below 4 tiles
 int co_pair_ds(co_ctx *c, int Mub) {
     if (Mub <= 0) return CO_OK;
-    if (co_cdiv(Mub, ST) >= 4) return pair_sym(c, Mub, 2);
-    return co_pair_fp64(c, Mub, 0);
+    const int nt = co_cdiv(Mub, ST), H = nt / 2, KC = SYM_KC, nchunk = co_cdiv(H + 1, KC);
+    if (nt < 4) return co_pair_fp64(c, Mub, 0);
+    const size_t gsz = (size_t)nchunk * nt * 2 * ST, asz = (size_t)(H > 0 ? H : 1) * nt * 2 * ST;
+    int rc = co_ensure_part(c, gsz + asz);
+    if (rc) return rc;
+    double *gpart = c->mb.part, *apart = c->mb.part + gsz;
+    co_prof_begin(c, 2);
+    k_pair_ds_sym<<<nt * nchunk, ST, 0, c->stream>>>(c->mb.pf_x, c->mb.pf_g, c->mb.pf_w,
+                                                     c->mb.pf_wl, nt, H, KC, gpart, apart);
+    co_prof_end(c);
+    k_sym_reduce<double><<<co_cdiv((long long)nt * ST, 256), 256, 0, c->stream>>>(
+        gpart, apart, nt, H, nchunk, ST, c->mb.pdot, (size_t)c->mb.cap);
+    c->launches += 2;
+    CO_CK(cudaGetLastError());
+    return CO_OK;
 }
 
 // ================================================================== batched
 //
 // Many independent ensembles in one persistent launch: the work items of all
-// Landau instances -- (instance, tile I, chunk of k) as in k_pair64_sym, with a
+// Landau instances -- (instance, tile I, chunk of k) as in the symmetric form above, with a
 // tile of T = 32 W markers -- are handed out through an atomic counter, so the
 // grid size and the tile shape are free parameters (chosen by the autotuner of
 // the batch engine). Items of instances whose solve has finished are skipped.
@@ -1434,7 +1365,7 @@ int co_batch_work_table(co_ctx *const *ctxs, const co_solver_state *const *state
         int nt = co_cdiv(N, T), H = nt / 2, nchunk = co_cdiv(H + 1, KC);
         size_t gsz = (size_t)nchunk * nt * 2 * T, asz = (size_t)(H > 0 ? H : 1) * nt * 2 * T;
         if (c->batch_landau) {
-            int rc = ensure_part(c, gsz + asz);
+            int rc = co_ensure_part(c, gsz + asz);
             if (rc) return -rc;
         }
         wk.px = c->mb.px;

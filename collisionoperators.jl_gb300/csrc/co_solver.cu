@@ -1364,7 +1364,10 @@ int co_step_defect_buffers(co_ctx *c, const co_opts *o, const co_defect_opts *do
         k_geff_store<<<co_cdiv(N, 256), 256, 0, c->stream>>>(N, b.dS, b.dv, b.w, c->st, gz, b.Gk);
         c->launches++;
         const int m64 = dopt->metric64 && stage == 0 && !ds;
-        int prec_pack = (stage == 1 || ds) ? CO_PREC_MIXED : (m64 ? CO_PREC_FP64 : CO_PREC_BOTH);
+        int prec_pack = stage == 1 ? CO_PREC_MIXED
+                        : ds         ? CO_PREC_MIXED_DS
+                        : m64        ? CO_PREC_FP64
+                                     : CO_PREC_BOTH;
         if ((rc = co_pack_landau(c, N, N, prec_pack, gz))) return rc;
         if (stage == 1) {
             rc = co_pair_fp32(c, N);
@@ -1710,7 +1713,7 @@ static int batch_pre(co_batch *B, int i, const co_opts *o, double S0i, double dt
                                b.v0, N, S0i, dt, b.r, nred);
     *nred = red_blocks(c, N);
     if ((rc = landau_geff_dev(c, o->use_gonzalez, b.v1, b.v0, N, S0i))) return rc;
-    return co_pack_landau(c, N, N, CO_PREC_FP64, o->use_gonzalez);
+    return co_pack_landau(c, N, N, CO_PREC_FP64, o->use_gonzalez, 1);
 }
 
 // fork: every aux stream waits for the main stream's work so far

@@ -1177,6 +1177,12 @@ int co_ensure_capacity(co_ctx *c, int N, int m) {
         if ((rc = grow(&b.pf_g, (size_t)cap))) return rc;
         if ((rc = grow(&b.pf_w, (size_t)cap))) return rc;
         if ((rc = grow(&b.pf_wl, (size_t)cap))) return rc;
+        if ((rc = grow(&b.fx_x, n2))) return rc;
+        if ((rc = grow(&b.fx_w, (size_t)cap))) return rc;
+        if ((rc = grow(&b.fx_g, (size_t)cap))) return rc;
+        if ((rc = grow(&b.pwn, (size_t)cap))) return rc;
+        if ((rc = grow(&b.unit, 4))) return rc;
+        if ((rc = grow(&b.gwmax, (size_t)cap / 256))) return rc;
         if ((rc = grow(&b.pdot, n2))) return rc;
         if ((rc = grow(&b.pA, 3 * (size_t)cap))) return rc;
         int nchunk = co_cdiv(cap, CO_CHUNK);
