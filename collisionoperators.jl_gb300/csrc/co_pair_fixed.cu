@@ -111,7 +111,7 @@ struct fixed_target {
 template <int NC, bool UNI>
 __device__ __forceinline__ void fixed_terms(fx64 S, const fx_limb &y3, fx_limb w,
                                             const fx_dist &d, fx64 (&T)[NC]) {
-    const fx_limb s = UNI ? fx_split_up<3>(S) : fx_split_up<4>(fx_mul(fx_split(S), w));
+    const fx_limb s = UNI ? fx_split_up<3>(S) : fx_split_up<1>(fx_mul(fx_split_up<3>(S), w));
     T[0] = fx_mul(s, d.d2);
     T[1] = fx_mul(s, d.d1);
     if (NC == 5) {
