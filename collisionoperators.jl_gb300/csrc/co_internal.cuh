@@ -160,7 +160,7 @@ struct co_ctx {
     struct co_prof *prof;
     unsigned long long maps64, maps32, mapsds;
     // batch membership (co_batch): marker count and whether the instance has a pair sum
-    int batch_N, batch_landau;
+    int batch_N, batch_landau, batch_member;
     int lb_two_pass;          // LB drift in two launches (capturable) instead of cooperative
     // bounded grid barrier of the cooperative LB kernel: polls before it gives
     // up with CO_ERR_TIMEOUT, and phantom blocks it waits for on top of the
@@ -220,7 +220,7 @@ int co_features_res_dev(co_ctx *c, int N, const double *r, double dt, float *X);
 int co_pair_fp64(co_ctx *c, int M, int with_metric);   // packed -> pdot (and pA)
 int co_pair_fp32(co_ctx *c, int M);                    // packed FP32 -> pdot
 int co_pair_ds(co_ctx *c, int M);                      // packed -> pdot, double-single form
-int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez, int batch = 0);
+int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez);
 int co_pack_plain(co_ctx *c, int N, int Mub, int precision, const double *x, const double *G);
 int co_unpack_A(co_ctx *c, int N, double *A);
 int co_metric32(co_ctx *c, int Mub);   // FP32 metric A (3 x ld in pA) from pf_x/pf_w
@@ -243,10 +243,13 @@ static inline int co_pack_mode(int precision) {
 }
 // Whether an FP64-accurate pair sum of up to Mub markers takes the fixed-point
 // kernel: from four 128-marker tiles on; below that the one-sided FP64 kernel's
-// single launch is as fast. The one-sided FP64 form also stays for CO_FLAG_ONESIDED.
+// single launch is as fast. The one-sided FP64 form also stays for CO_FLAG_ONESIDED,
+// and the batch engine keeps the FP64 form: a solve that stagnates returns an iterate
+// that round-off decides, and in a sample of batches 3 of 14 held such an instance,
+// whose result moved by 1e-6 to 1e-4 under the fixed-point sums.
 static inline int co_use_fixed(const co_ctx *c, int Mub, int precision) {
     return (precision == CO_PREC_FP64 || precision == CO_PREC_BOTH) && c->pair_symmetric &&
-           co_cdiv(Mub, 128) >= 4;
+           !c->batch_member && co_cdiv(Mub, 128) >= 4;
 }
 // operands of the fixed-point pair sum, as the kernels take them
 struct co_fixed_ops {

@@ -9,7 +9,7 @@
 //
 // The reference's Float64 path runs on the fixed-point kernels of co_pair_fixed.cu;
 // the FP64 arithmetic below serves the one-sided kernels (CO_FLAG_ONESIDED, fewer
-// than 385 markers) and the batched one. On GB300 FP64 issues at 1/64 of the FP32
+// than 385 markers) and the batch engine. On GB300 FP64 issues at 1/64 of the FP32
 // rate, so the per-pair FP64 instruction count is what sets its time. The pair body
 // is 20 FP64 instructions:
 //   d (2), |d|^2 (2), 1/|d| refinement (5), G difference (2), d.g (2),
@@ -345,6 +345,71 @@ __device__ __forceinline__ void pair_u64(double d1, double d2, double g1, double
 
 __device__ __forceinline__ bool sym_skip(int nt, int H, int I, int k) {
     return k > 0 && (nt & 1) == 0 && k == H && I >= nt / 2;
+}
+
+// The explicit predictor of a batch instance; the instances' iterations run the
+// same arithmetic in k_pair64_sym_batch.
+__global__ void __launch_bounds__(ST)
+k_pair64_sym(const double2 *__restrict__ px, const double2 *__restrict__ pg,
+             const double *__restrict__ pw, int nt, int H, int KC,
+             double *__restrict__ gpart, double *__restrict__ apart) {
+    __shared__ double2 sx[ST], sg[ST];
+    __shared__ double sw[ST];
+    __shared__ double2 sacc[ST];
+    const int I = blockIdx.x % nt, chunk = blockIdx.x / nt;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const double2 xg = px[I * ST + tid], Gg = pg[I * ST + tid];
+    const double wg = pw[I * ST + tid];
+    double ga1 = 0.0, ga2 = 0.0;
+    const int k0 = chunk * KC, k1 = min(H + 1, k0 + KC);
+    for (int k = k0; k < k1; k++) {
+        if (sym_skip(nt, H, I, k)) continue;
+        const int J = (I + k) % nt;
+        __syncthreads();
+        sx[tid] = px[J * ST + tid];
+        sg[tid] = pg[J * ST + tid];
+        sw[tid] = pw[J * ST + tid];
+        sacc[tid] = make_double2(0.0, 0.0);
+        __syncthreads();
+        if (k == 0) {  // diagonal tile: ordered pairs, self excluded by the guard
+#pragma unroll 4
+            for (int a = 0; a < ST; a++) {
+                double u1, u2;
+                double2 xa = sx[a], Ga = sg[a];
+                pair_u64(xg.x - xa.x, xg.y - xa.y, Ga.x - Gg.x, Ga.y - Gg.y, u1, u2);
+                ga1 = fma(sw[a], u1, ga1);
+                ga2 = fma(sw[a], u2, ga2);
+            }
+            continue;
+        }
+        for (int r = 0; r < 4; r++) {
+            const int base = ((warp + r) & 3) * 32;
+            double2 a0 = sacc[base + lane];
+            double a1 = a0.x, a2 = a0.y;
+#pragma unroll 4
+            for (int q = 0; q < 32; q++) {
+                const int ai = base + ((lane + q) & 31);
+                double2 xa = sx[ai], Ga = sg[ai];
+                double wa = sw[ai];
+                double u1, u2;
+                pair_u64(xg.x - xa.x, xg.y - xa.y, Ga.x - Gg.x, Ga.y - Gg.y, u1, u2);
+                ga1 = fma(wa, u1, ga1);
+                ga2 = fma(wa, u2, ga2);
+                a1 = fma(-wg, u1, a1);
+                a2 = fma(-wg, u2, a2);
+                a1 = __shfl_sync(0xffffffffu, a1, (lane + 1) & 31);
+                a2 = __shfl_sync(0xffffffffu, a2, (lane + 1) & 31);
+            }
+            sacc[base + lane] = make_double2(a1, a2);
+            __syncthreads();
+        }
+        double *ap = apart + ((size_t)(k - 1) * nt + J) * 2 * ST;
+        ap[tid] = sacc[tid].x;
+        ap[ST + tid] = sacc[tid].y;
+    }
+    double *gp = gpart + ((size_t)chunk * nt + I) * 2 * ST;
+    gp[tid] = ga1;
+    gp[ST + tid] = ga2;
 }
 
 // FP32 body on head/tail operands: returns the unweighted term u
@@ -1142,10 +1207,31 @@ int co_ensure_part(co_ctx *c, size_t n) {
     return CO_OK;
 }
 
+#define SYM_KC 8
+
+// FP64 symmetric pair sum on the padded operands (batch instances)
+static int pair64_sym(co_ctx *c, int Mub) {
+    const int nt = co_cdiv(Mub, ST), H = nt / 2, KC = SYM_KC, nchunk = co_cdiv(H + 1, KC);
+    const size_t gsz = (size_t)nchunk * nt * 2 * ST, asz = (size_t)(H > 0 ? H : 1) * nt * 2 * ST;
+    int rc = co_ensure_part(c, gsz + asz);
+    if (rc) return rc;
+    double *gpart = c->mb.part, *apart = c->mb.part + gsz;
+    co_prof_begin(c, 1);
+    k_pair64_sym<<<nt * nchunk, ST, 0, c->stream>>>(c->mb.px, c->mb.pg, c->mb.pw, nt, H, KC, gpart,
+                                                    apart);
+    co_prof_end(c);
+    k_sym_reduce<double><<<co_cdiv((long long)nt * ST, 256), 256, 0, c->stream>>>(
+        gpart, apart, nt, H, nchunk, ST, c->mb.pdot, (size_t)c->mb.cap);
+    c->launches += 2;
+    CO_CK(cudaGetLastError());
+    return CO_OK;
+}
+
 // M is an upper bound (N); the true count sits at cstart[n_el] on the device.
 int co_pair_fp64(co_ctx *c, int Mub, int with_metric) {
     if (Mub <= 0) return CO_OK;
     if (co_use_fixed(c, Mub, CO_PREC_FP64)) return co_pair_fixed_sum(c, Mub, with_metric, 1);
+    if (!with_metric && c->pair_symmetric && co_cdiv(Mub, ST) >= 4) return pair64_sym(c, Mub);
     const int *Mp = c->mb.cstart + c->n_el;
     size_t ld = (size_t)c->mb.cap;
     int split = choose_split(c, Mub, PAIR_TPB, c->pair_split_fp64);
@@ -1184,8 +1270,6 @@ int co_pair_fp64(co_ctx *c, int Mub, int with_metric) {
     CO_CK(cudaGetLastError());
     return CO_OK;
 }
-
-#define SYM_KC 8
 
 // FP32 symmetric pair sum: two targets per thread on 256-marker tiles (Mpad is a
 // multiple of 256 and the tile count has been checked by the caller)
@@ -1257,8 +1341,7 @@ int co_pack_plain(co_ctx *c, int N, int Mub, int precision, const double *x, con
     return co_use_fixed(c, Mub, precision) ? co_pair_fixed_pack(c, Mub, Mpad / 256) : CO_OK;
 }
 
-// batch != 0: the operands of the batched FP64 kernel only
-int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez, int batch) {
+int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez) {
     if (Mub <= 0) return CO_OK;
     const int *Mp = c->mb.cstart + c->n_el;
     co_bufs &b = c->mb;
@@ -1268,8 +1351,7 @@ int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez, int b
                                                      pack_out(c));
     c->launches++;
     CO_CK(cudaGetLastError());
-    return !batch && co_use_fixed(c, Mub, precision) ? co_pair_fixed_pack(c, Mub, Mpad / 256)
-                                                     : CO_OK;
+    return co_use_fixed(c, Mub, precision) ? co_pair_fixed_pack(c, Mub, Mpad / 256) : CO_OK;
 }
 
 int co_unpack_update(co_ctx *c, int N, double dt, double *Gv, const double *v0,

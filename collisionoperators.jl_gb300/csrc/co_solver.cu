@@ -1655,6 +1655,7 @@ extern "C" int co_batch_create(const co_batch_instance *inst, int n, int n_quad,
         cudaFree(c->st);
         c->st = B->st_all + i;
         c->lb_two_pass = 1;
+        c->batch_member = 1;
         c->batch_N = d.N;
         c->batch_landau = d.model == CO_MODEL_LANDAU;
         B->ctx.push_back(c);
@@ -1713,7 +1714,7 @@ static int batch_pre(co_batch *B, int i, const co_opts *o, double S0i, double dt
                                b.v0, N, S0i, dt, b.r, nred);
     *nred = red_blocks(c, N);
     if ((rc = landau_geff_dev(c, o->use_gonzalez, b.v1, b.v0, N, S0i))) return rc;
-    return co_pack_landau(c, N, N, CO_PREC_FP64, o->use_gonzalez, 1);
+    return co_pack_landau(c, N, N, CO_PREC_FP64, o->use_gonzalez);
 }
 
 // fork: every aux stream waits for the main stream's work so far
