@@ -178,6 +178,7 @@ __device__ __forceinline__ void fixed_group(fixed_smem<W, NC> &sm, const co_fixe
         }
     }
     if (SRC) {
+        __syncwarp();   // close pairs of other lanes have added to this lane's sources
         const int k = grp * 32 + lane;
 #pragma unroll
         for (int i = 0; i < NC; i++) sm.acc[i][k] = fma(tf[i > 1], fx_to_double(b[i]), sm.acc[i][k]);
