@@ -614,12 +614,11 @@ k_pair32_sym(const float4 *__restrict__ pfx, const float4 *__restrict__ pfg,
 // The same symmetric pair sum in double-single arithmetic: every value is an
 // unevaluated sum hi + lo of two FP32 numbers (about 44 significant bits), built
 // from the error-free transformations of Dekker (1971) and Knuth (TAOCP vol. 2):
-// two_sum (6 adds), fast_two_sum (3), two_prod via FMA (2). The intrinsics
+// two_sum (6 adds), fast_two_sum (3), two_prod via FMA (2). The scalar form serves the
+// diagonal tiles, the packed form below it all other tile pairs. The intrinsics
 // __fadd_rn/__fsub_rn/__fmul_rn/__fmaf_rn keep the compiler from contracting
-// these sequences. 1/|d| is one Newton step from the MUFU seed. Each unordered
-// pair (both orders) costs about 190 FP32 instructions against 20 FP64
-// instructions of the FP64 form, i.e. about 7x less issue time on a part whose
-// FP32:FP64 rate is 64:1, at ~1e-13 relative accuracy per term; momentum stays
+// these sequences. Each unordered pair (both orders) costs 137 FP32 operations at
+// ~1e-13 relative accuracy per term; momentum stays
 // exact to the accumulation round-off because each pair's term is computed once
 // and added with both signs. Used for the FP64 stage of the mixed precision form.
 struct dsf {
@@ -635,18 +634,6 @@ __device__ __forceinline__ dsf ds_two_sum(float a, float b) {
 __device__ __forceinline__ dsf ds_fast(float a, float b) {
     float s = __fadd_rn(a, b);
     return {s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ dsf ds_add(dsf a, dsf b) {
-    dsf s = ds_two_sum(a.h, b.h);
-    return ds_fast(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
-}
-__device__ __forceinline__ dsf ds_sub(dsf a, dsf b) { return ds_add(a, {-b.h, -b.l}); }
-__device__ __forceinline__ dsf ds_mul(dsf a, dsf b) {
-    float p = __fmul_rn(a.h, b.h);
-    float e = __fmaf_rn(a.h, b.h, -p);
-    e = __fmaf_rn(a.h, b.l, e);
-    e = __fmaf_rn(a.l, b.h, e);
-    return ds_fast(p, e);
 }
 // Unnormalised double-single values: an intermediate that only feeds a
 // product or a sum is kept as an exact pair (h, l) whose l may exceed
@@ -722,131 +709,242 @@ __device__ __forceinline__ void pair_s_ds(const float4 &xg, const float4 &Gg, co
     if (!ok) s = {0.f, 0.f};
 }
 
-// Tile pairs whose 2 x 128 markers all carry one weight w0 (the common case:
-// equal-weight markers) take the unweighted loop: the terms s (d2, -d1) are
-// summed without the per-pair weight products and w0 multiplies the FP64 fold
-// (16 of ~190 instructions per pair saved). A block vote on the loaded tile
-// decides per tile pair; padding (weight 0) and unequal weights take the
-// weighted loop.
-__global__ void __launch_bounds__(ST)
+// Double-single values of two tile pairs in the halves of packed registers, operation
+// for operation as above: each half is rounded as the scalar form rounds it. A product
+// whose value enters a sum is an FMA with a -0 the compiler cannot see (nz), because a
+// packed product and the sum it enters would be contracted into one FMA.
+struct ds2 {
+    f32x2 h, l;
+};
+__device__ __forceinline__ ds2 ds2_norm(f32x2 h, f32x2 l) {
+    const f32x2 s = add2(h, l);
+    return {s, sub2(l, sub2(s, h))};
+}
+// a - b, unnormalised
+__device__ __forceinline__ ds2 ds2_sub(ds2 a, ds2 b) {
+    const f32x2 s = sub2(a.h, b.h);
+    const f32x2 bb = sub2(s, a.h);
+    const f32x2 e = sub2(sub2(a.h, sub2(s, bb)), add2(b.h, bb));
+    return {s, add2(e, sub2(a.l, b.l))};
+}
+__device__ __forceinline__ ds2 ds2_sqr(ds2 a, f32x2 nz) {
+    const f32x2 p = fma2(a.h, a.h, nz);
+    return {p, fma2(add2(a.h, a.h), a.l, fma2(a.h, a.h, neg2(p)))};
+}
+// a b, unnormalised; SUM: the head enters a sum
+template <bool SUM>
+__device__ __forceinline__ ds2 ds2_mul(ds2 a, ds2 b, f32x2 nz) {
+    const f32x2 p = SUM ? fma2(a.h, b.h, nz) : mul2(a.h, b.h);
+    f32x2 e = fma2(a.h, b.h, neg2(p));
+    e = fma2(a.h, b.l, e);
+    e = fma2(a.l, b.h, e);
+    return {p, e};
+}
+__device__ __forceinline__ void ds2_acc(ds2 &acc, ds2 x) {
+    const f32x2 s = add2(acc.h, x.h);
+    const f32x2 bb = sub2(s, acc.h);
+    const f32x2 e = add2(sub2(acc.h, sub2(s, bb)), sub2(x.h, bb));
+    acc.h = s;
+    acc.l = add2(acc.l, add2(x.l, e));
+}
+// pair_s_ds of both halves; the sources' operands as {h of both, l of both}
+__device__ __forceinline__ void pair_s_ds2(const ds2 (&xg)[2], const ds2 (&Gg)[2], ds2 xa1, ds2 xa2,
+                                           ds2 Ga1, ds2 Ga2, f32x2 nz, ds2 &d1, ds2 &d2, ds2 &s) {
+    d1 = ds2_sub(xg[0], xa1);
+    d1 = ds2_norm(d1.h, d1.l);
+    d2 = ds2_sub(xg[1], xa2);
+    d2 = ds2_norm(d2.h, d2.l);
+    const ds2 q1 = ds2_sqr(d1, nz), q2 = ds2_sqr(d2, nz);
+    const f32x2 rh = add2(q1.h, q2.h);
+    const f32x2 rb = sub2(rh, q1.h);
+    const f32x2 re = add2(sub2(q1.h, sub2(rh, rb)), sub2(q2.h, rb));
+    const f32x2 rl = add2(re, add2(q1.l, q2.l));
+    const float ra = lo2(rh), rc = hi2(rh);
+    const f32x2 y0 = pack2(rsqrt_normal(ra), rsqrt_normal(rc));
+    const f32x2 p2 = mul2(y0, y0);
+    const f32x2 e2 = fma2(y0, y0, neg2(p2));
+    const f32x2 q = fma2(rh, p2, nz);
+    f32x2 qe = fma2(rh, p2, neg2(q));
+    qe = fma2(rh, e2, qe);
+    qe = fma2(rl, p2, qe);
+    const f32x2 e = sub2(sub2(dup2(1.0f), q), qe);
+    const f32x2 p3 = mul2(p2, y0);
+    f32x2 e3 = fma2(p2, y0, neg2(p3));
+    e3 = fma2(e2, y0, e3);
+    const f32x2 corr = mul2(e, fma2(dup2(1.875f), e, dup2(1.5f)));
+    const ds2 y3 = {p3, fma2(p3, corr, e3)};
+    ds2 g1 = ds2_sub(Ga1, Gg[0]);
+    g1 = ds2_norm(g1.h, g1.l);
+    ds2 g2 = ds2_sub(Ga2, Gg[1]);
+    g2 = ds2_norm(g2.h, g2.l);
+    ds2 c = ds2_sub(ds2_mul<true>(g1, d2, nz), ds2_mul<true>(g2, d1, nz));
+    c = ds2_norm(c.h, c.l);
+    s = ds2_mul<false>(c, y3, nz);
+    // the guard acts on s alone: what a discarded half computed does not spread
+    const bool oka = ra >= 1e-24f, okc = rc >= 1e-24f;
+    s.h = pack2(oka ? lo2(s.h) : 0.f, okc ? hi2(s.h) : 0.f);
+    s.l = pack2(oka ? lo2(s.l) : 0.f, okc ? hi2(s.l) : 0.f);
+}
+
+struct ds_smem {
+    ulonglong2 xh[ST], xl[ST], gh[ST], gl[ST];   // {component 1 of both tiles, component 2}
+    ulonglong2 w[ST];                            // weights {heads, tails}
+    ulonglong2 a1[ST], a2[ST];                   // source sums {heads, tails}
+};
+
+// Warp w's targets against the two tiles in sm, off the diagonal: in round r it meets
+// the sources of group (w + r) mod 4, whose sums rotate with the lanes and pass from
+// warp to warp through sm between rounds. UNI: the unweighted terms s (d2, -d1) on
+// both sides. The second components are summed without their sign.
+template <bool UNI>
+__device__ __forceinline__ void ds_tiles(ds_smem &sm, const ds2 (&xg)[2], const ds2 (&Gg)[2], ds2 wg,
+                                         f32x2 nz, int lane, int warp, ds2 &ga1, ds2 &ga2) {
+#pragma unroll 1
+    for (int r = 0; r < 4; r++) {
+        const int base = ((warp + r) & 3) * 32;
+        ds2 a1 = {sm.a1[base + lane].x, sm.a1[base + lane].y};
+        ds2 a2 = {sm.a2[base + lane].x, sm.a2[base + lane].y};
+#pragma unroll 1
+        for (int q = 0; q < 32; q++) {
+            const int ai = base + ((lane + q) & 31);
+            const ulonglong2 xh = sm.xh[ai], xl = sm.xl[ai], gh = sm.gh[ai], gl = sm.gl[ai];
+            ds2 d1, d2, s;
+            pair_s_ds2(xg, Gg, {xh.x, xl.x}, {xh.y, xl.y}, {gh.x, gl.x}, {gh.y, gl.y}, nz, d1, d2, s);
+            if (UNI) {
+                const ds2 t1 = ds2_mul<true>(s, d2, nz), t2 = ds2_mul<true>(s, d1, nz);
+                ds2_acc(ga1, t1);
+                ds2_acc(ga2, t2);
+                ds2_acc(a1, t1);
+                ds2_acc(a2, t2);
+            } else {
+                const ulonglong2 wa = sm.w[ai];
+                const ds2 ws = ds2_mul<false>({wa.x, wa.y}, s, nz);   // w_a s
+                const ds2 wn = ds2_mul<false>(wg, s, nz);             // -w_g s
+                ds2_acc(ga1, ds2_mul<true>(ws, d2, nz));
+                ds2_acc(ga2, ds2_mul<true>(ws, d1, nz));
+                ds2_acc(a1, ds2_mul<true>(wn, d2, nz));
+                ds2_acc(a2, ds2_mul<true>(wn, d1, nz));
+            }
+            const int src = (lane + 1) & 31;
+            a1.h = __shfl_sync(0xffffffffu, a1.h, src);
+            a1.l = __shfl_sync(0xffffffffu, a1.l, src);
+            a2.h = __shfl_sync(0xffffffffu, a2.h, src);
+            a2.l = __shfl_sync(0xffffffffu, a2.l, src);
+        }
+        a1 = ds2_norm(a1.h, a1.l);
+        a2 = ds2_norm(a2.h, a2.l);
+        ga1 = ds2_norm(ga1.h, ga1.l);
+        ga2 = ds2_norm(ga2.h, ga2.l);
+        sm.a1[base + lane] = make_ulonglong2(a1.h, a1.l);
+        sm.a2[base + lane] = make_ulonglong2(a2.h, a2.l);
+        __syncthreads();
+    }
+}
+
+// Two consecutive tile pairs of a row in the halves of packed registers, as in
+// k_pair32_sym. Tile pairs whose 2 x 128 markers all carry one weight w0 (the common
+// case: equal-weight markers) take the unweighted loop: the terms s (d2, -d1) are
+// summed without the per-pair weight products and w0 multiplies the FP64 fold. A block
+// vote on the loaded tiles decides; padding (weight 0) and unequal weights take the
+// weighted loop. Two tiles that differ in this take a pass each, the first tile's first.
+// 137 FP32 operations a pair in packed instructions. What bounds it is the FMA pipe,
+// which issues packed operations with three distinct register operands at two thirds of
+// its rate: 2.35 of the 2.56 clocks that two pairs take on an SM. 90 registers, five
+// blocks per SM (six: 1 % slower). Bit-identical to the scalar form it replaces: 131,072
+// markers 41.7 -> 37.7 ms a map, 47.9 -> 43.2 with unequal weights.
+__global__ void __launch_bounds__(ST, 5)
 k_pair_ds_sym(const float4 *__restrict__ pfx, const float4 *__restrict__ pfg,
               const float *__restrict__ pfw, const float *__restrict__ pfwl, int nt, int H,
-              int KC, double *__restrict__ gpart, double *__restrict__ apart) {
-    __shared__ float4 sx[ST], sg[ST];
-    __shared__ float2 sw[ST];
-    __shared__ float4 sacc[ST];  // {a1.h, a1.l, a2.h, a2.l}
+              int KC, double *__restrict__ gpart, double *__restrict__ apart, f32x2 nz) {
+    __shared__ ds_smem sm;
     const int I = blockIdx.x % nt, chunk = blockIdx.x / nt;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float4 xg = pfx[I * ST + tid], Gg = pfg[I * ST + tid];
-    const dsf wg = {pfw[I * ST + tid], pfwl[I * ST + tid]};
     const float2 w0 = make_float2(pfw[I * ST], pfwl[I * ST]);
     const double w0d = (double)w0.x + (double)w0.y;
-    const bool own_same = wg.h == w0.x && wg.l == w0.y && w0.x != 0.f;
-    dsf ga1 = {0.f, 0.f}, ga2 = {0.f, 0.f};
     double gd1 = 0.0, gd2 = 0.0;
     const int k0 = chunk * KC, k1 = min(H + 1, k0 + KC);
-    for (int k = k0; k < k1; k++) {
-        if (sym_skip(nt, H, I, k)) continue;
-        const int J = (I + k) % nt;
-        __syncthreads();
-        sx[tid] = pfx[J * ST + tid];
-        sg[tid] = pfg[J * ST + tid];
-        const float2 wa = make_float2(pfw[J * ST + tid], pfwl[J * ST + tid]);
-        sw[tid] = wa;
-        sacc[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const bool uni =
-            __syncthreads_and(own_same && wa.x == w0.x && wa.y == w0.y) != 0;
-        if (k == 0) {
-            if (uni) {
-                for (int a = 0; a < ST; a++) {
-                    dsf d1, d2, sp;
-                    pair_s_ds(xg, Gg, sx[a], sg[a], d1, d2, sp);
-                    const dsf t2 = ds_mul_u(sp, d1);
-                    ds_acc(ga1, ds_mul_u(sp, d2));
-                    ds_acc(ga2, {-t2.h, -t2.l});
-                    if ((a & 31) == 31) {
-                        ga1 = ds_norm(ga1);
-                        ga2 = ds_norm(ga2);
-                    }
-                }
-            } else {
-                for (int a = 0; a < ST; a++) {
-                    dsf d1, d2, sp;
-                    pair_s_ds(xg, Gg, sx[a], sg[a], d1, d2, sp);
-                    const dsf ws = ds_mul_u({sw[a].x, sw[a].y}, sp);
-                    ds_acc(ga1, ds_mul_u(ws, d2));
-                    ds_acc(ga2, ds_mul_u(ws, {-d1.h, -d1.l}));
-                    if ((a & 31) == 31) {
-                        ga1 = ds_norm(ga1);
-                        ga2 = ds_norm(ga2);
-                    }
-                }
+    int k = k0;
+    const float4 x = pfx[I * ST + tid], g = pfg[I * ST + tid];
+    const dsf w = {pfw[I * ST + tid], pfwl[I * ST + tid]};
+    const bool own_same = w.h == w0.x && w.l == w0.y && w0.x != 0.f;
+    if (k == 0) {   // diagonal tile: ordered pairs, self excluded by the guard
+        float4 *sx = reinterpret_cast<float4 *>(sm.xh), *sg = reinterpret_cast<float4 *>(sm.gh);
+        float2 *sw = reinterpret_cast<float2 *>(sm.w);
+        sx[tid] = x;
+        sg[tid] = g;
+        sw[tid] = make_float2(w.h, w.l);
+        const bool uni = __syncthreads_and(own_same) != 0;
+        dsf t1 = {0.f, 0.f}, t2 = {0.f, 0.f};
+        for (int a = 0; a < ST; a++) {
+            dsf d1, d2, s;
+            pair_s_ds(x, g, sx[a], sg[a], d1, d2, s);
+            if (!uni) s = ds_mul_u({sw[a].x, sw[a].y}, s);
+            ds_acc(t1, ds_mul_u(s, d2));
+            ds_acc(t2, ds_mul_u(s, {-d1.h, -d1.l}));
+            if ((a & 31) == 31) {
+                t1 = ds_norm(t1);
+                t2 = ds_norm(t2);
             }
-        } else {
-            for (int r = 0; r < 4; r++) {
-                const int base = ((warp + r) & 3) * 32;
-                float4 a0 = sacc[base + lane];
-                dsf a1 = {a0.x, a0.y}, a2 = {a0.z, a0.w};
-                if (uni) {
-                    // target += s (d2, -d1); source accumulates the same terms,
-                    // its factor -w0 applied at the write-out
-#pragma unroll 2
-                    for (int q = 0; q < 32; q++) {
-                        const int ai = base + ((lane + q) & 31);
-                        dsf d1, d2, sp;
-                        pair_s_ds(xg, Gg, sx[ai], sg[ai], d1, d2, sp);
-                        const dsf t1 = ds_mul_u(sp, d2);
-                        const dsf t2 = ds_mul_u(sp, d1);
-                        const dsf nt2 = {-t2.h, -t2.l};
-                        ds_acc(ga1, t1);
-                        ds_acc(ga2, nt2);
-                        ds_acc(a1, t1);
-                        ds_acc(a2, nt2);
-                        const int src = (lane + 1) & 31;
-                        a1.h = __shfl_sync(0xffffffffu, a1.h, src);
-                        a1.l = __shfl_sync(0xffffffffu, a1.l, src);
-                        a2.h = __shfl_sync(0xffffffffu, a2.h, src);
-                        a2.l = __shfl_sync(0xffffffffu, a2.l, src);
-                    }
-                } else {
-#pragma unroll 2
-                    for (int q = 0; q < 32; q++) {
-                        const int ai = base + ((lane + q) & 31);
-                        dsf d1, d2, sp;
-                        pair_s_ds(xg, Gg, sx[ai], sg[ai], d1, d2, sp);
-                        const dsf ws = ds_mul_u({sw[ai].x, sw[ai].y}, sp);   // w_a s
-                        const dsf wn = ds_mul_u({-wg.h, -wg.l}, sp);         // -w_g s
-                        const dsf nd1 = {-d1.h, -d1.l};
-                        ds_acc(ga1, ds_mul_u(ws, d2));
-                        ds_acc(ga2, ds_mul_u(ws, nd1));
-                        ds_acc(a1, ds_mul_u(wn, d2));
-                        ds_acc(a2, ds_mul_u(wn, nd1));
-                        const int src = (lane + 1) & 31;
-                        a1.h = __shfl_sync(0xffffffffu, a1.h, src);
-                        a1.l = __shfl_sync(0xffffffffu, a1.l, src);
-                        a2.h = __shfl_sync(0xffffffffu, a2.h, src);
-                        a2.l = __shfl_sync(0xffffffffu, a2.l, src);
-                    }
-                }
-                a1 = ds_norm(a1);
-                a2 = ds_norm(a2);
-                ga1 = ds_norm(ga1);
-                ga2 = ds_norm(ga2);
-                sacc[base + lane] = make_float4(a1.h, a1.l, a2.h, a2.l);
+        }
+        const double tf = uni ? w0d : 1.0;
+        gd1 += tf * ((double)t1.h + (double)t1.l);
+        gd2 += tf * ((double)t2.h + (double)t2.l);
+        k = 1;
+    }
+    const ds2 xg[2] = {{dup2(x.x), dup2(x.z)}, {dup2(x.y), dup2(x.w)}};
+    const ds2 Gg[2] = {{dup2(g.x), dup2(g.z)}, {dup2(g.y), dup2(g.w)}};
+    const ds2 wg = {dup2(-w.h), dup2(-w.l)};
+    while (k < k1) {
+        if (sym_skip(nt, H, I, k)) break;   // k = H, the last one
+        bool two;
+        const int kn = next_pair(nt, H, I, k, k1, two);
+        const int J[2] = {(I + k) % nt, (I + k + 1) % nt};
+        __syncthreads();
+        const float4 xa = pfx[J[0] * ST + tid], ga = pfg[J[0] * ST + tid];
+        const float2 wa = make_float2(pfw[J[0] * ST + tid], pfwl[J[0] * ST + tid]);
+        float4 xb = make_float4(1e3f, 1e3f, 0.f, 0.f), gb = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 wb = wa;
+        if (two) {
+            xb = pfx[J[1] * ST + tid];
+            gb = pfg[J[1] * ST + tid];
+            wb = make_float2(pfw[J[1] * ST + tid], pfwl[J[1] * ST + tid]);
+        }
+        sm.xh[tid] = make_ulonglong2(pack2(xa.x, xb.x), pack2(xa.y, xb.y));
+        sm.xl[tid] = make_ulonglong2(pack2(xa.z, xb.z), pack2(xa.w, xb.w));
+        sm.gh[tid] = make_ulonglong2(pack2(ga.x, gb.x), pack2(ga.y, gb.y));
+        sm.gl[tid] = make_ulonglong2(pack2(ga.z, gb.z), pack2(ga.w, gb.w));
+        sm.w[tid] = make_ulonglong2(pack2(wa.x, wb.x), pack2(wa.y, wb.y));
+        sm.a1[tid] = sm.a2[tid] = make_ulonglong2(0, 0);
+        const bool ua = __syncthreads_and(own_same && wa.x == w0.x && wa.y == w0.y) != 0;
+        const bool ub = __syncthreads_and(own_same && wb.x == w0.x && wb.y == w0.y) != 0;
+        for (int pass = 0; pass < (ua == ub ? 1 : 2); pass++) {
+            const bool uni = pass ? ub : ua;
+            ds2 t1 = {0, 0}, t2 = {0, 0};
+            if (pass) {
+                sm.a1[tid] = sm.a2[tid] = make_ulonglong2(0, 0);
                 __syncthreads();
             }
-            double *ap = apart + ((size_t)(k - 1) * nt + J) * 2 * ST;
-            float4 v = sacc[tid];
-            const double sf = uni ? -w0d : 1.0;
-            ap[tid] = sf * ((double)v.x + (double)v.y);
-            ap[ST + tid] = sf * ((double)v.z + (double)v.w);
+            if (uni) ds_tiles<true>(sm, xg, Gg, wg, nz, lane, warp, t1, t2);
+            else ds_tiles<false>(sm, xg, Gg, wg, nz, lane, warp, t1, t2);
+            // fold each tile pair's double-single sums into FP64
+            const double tf = uni ? w0d : 1.0, sf = uni ? -w0d : 1.0;
+            const ulonglong2 v1 = sm.a1[tid], v2 = sm.a2[tid];
+            if (pass == 0) {
+                double *ap = apart + ((size_t)(k - 1) * nt + J[0]) * 2 * ST;
+                gd1 += tf * ((double)lo2(t1.h) + (double)lo2(t1.l));
+                gd2 -= tf * ((double)lo2(t2.h) + (double)lo2(t2.l));
+                ap[tid] = sf * ((double)lo2(v1.x) + (double)lo2(v1.y));
+                ap[ST + tid] = -sf * ((double)lo2(v2.x) + (double)lo2(v2.y));
+            }
+            if (two && (pass == 1 || ua == ub)) {
+                double *bp = apart + ((size_t)k * nt + J[1]) * 2 * ST;
+                gd1 += tf * ((double)hi2(t1.h) + (double)hi2(t1.l));
+                gd2 -= tf * ((double)hi2(t2.h) + (double)hi2(t2.l));
+                bp[tid] = sf * ((double)hi2(v1.x) + (double)hi2(v1.y));
+                bp[ST + tid] = -sf * ((double)hi2(v2.x) + (double)hi2(v2.y));
+            }
         }
-        // fold the tile pair's target-side double-single sum into FP64
-        const double tf = uni ? w0d : 1.0;
-        gd1 += tf * ((double)ga1.h + (double)ga1.l);
-        gd2 += tf * ((double)ga2.h + (double)ga2.l);
-        ga1 = {0.f, 0.f};
-        ga2 = {0.f, 0.f};
+        k = kn;
     }
     double *gp = gpart + ((size_t)chunk * nt + I) * 2 * ST;
     gp[tid] = gd1;
@@ -1414,7 +1512,8 @@ int co_pair_ds(co_ctx *c, int Mub) {
     double *gpart = c->mb.part, *apart = c->mb.part + gsz;
     co_prof_begin(c, 2);
     k_pair_ds_sym<<<nt * nchunk, ST, 0, c->stream>>>(c->mb.pf_x, c->mb.pf_g, c->mb.pf_w,
-                                                     c->mb.pf_wl, nt, H, KC, gpart, apart);
+                                                     c->mb.pf_wl, nt, H, KC, gpart, apart,
+                                                     0x8000000080000000ull);
     co_prof_end(c);
     k_sym_reduce<double><<<co_cdiv((long long)nt * ST, 256), 256, 0, c->stream>>>(
         gpart, apart, nt, H, nchunk, ST, c->mb.pdot, (size_t)c->mb.cap);
