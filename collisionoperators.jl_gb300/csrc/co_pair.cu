@@ -1236,7 +1236,7 @@ k_unpack_update(const int *__restrict__ inv, int N, const double *__restrict__ p
                 double dt, const double *__restrict__ v0, double *__restrict__ Gv,
                 double *__restrict__ dotv, const double *__restrict__ v1, double *__restrict__ r,
                 double *__restrict__ red) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     double sr = 0.0, sv = 0.0;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < N; a += gridDim.x * blockDim.x) {
         int p = inv[a];
@@ -1264,11 +1264,11 @@ k_unpack_update(const int *__restrict__ inv, int N, const double *__restrict__ p
         }
     }
     if (red) {
-        double a = co_block_sum(sr, sh);
-        double b = co_block_sum(sv, sh);
+        double s[2] = {sr, sv};
+        co_block_sums<2>(s, sh);
         if (threadIdx.x == 0) {
-            red[blockIdx.x * 2 + 0] = a;
-            red[blockIdx.x * 2 + 1] = b;
+            red[blockIdx.x * 2 + 0] = s[0];
+            red[blockIdx.x * 2 + 1] = s[1];
         }
     }
 }

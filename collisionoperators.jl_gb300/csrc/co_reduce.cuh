@@ -23,6 +23,32 @@ __device__ __forceinline__ double co_block_sum(double v, double *sh /* >= 32 */)
     return r;
 }
 
+// co_block_sum of V values at once, each in co_block_sum's order: the V shuffle trees
+// overlap and share three barriers instead of taking four each, one after another
+// (small launches wait on these chains). sh: >= 32 V doubles.
+template <int V>
+__device__ __forceinline__ void co_block_sums(double (&v)[V], double *sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < V; i++) v[i] += __shfl_down_sync(0xffffffffu, v[i], o);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    __syncthreads();
+    if (lane == 0)
+#pragma unroll
+        for (int i = 0; i < V; i++) sh[32 * i + warp] = v[i];
+    __syncthreads();
+    for (int i = warp; i < V; i += nw) {
+        double s = lane < nw ? sh[32 * i + lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        __syncwarp();
+        if (lane == 0) sh[32 * i] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < V; i++) v[i] = sh[32 * i];
+}
+
 // s += v[i0], v[i0 + step], ... (i < n) in that order. The loads are issued
 // eight at a time ahead of the adds, so a thread waits for one L2 round trip
 // per eight terms rather than per term; the additions keep their order.

@@ -55,12 +55,15 @@ static const char *prec_name(int p) {
 __global__ void __launch_bounds__(256)
 k_lambda(const double *__restrict__ red, int nred, co_solver_state *st, double S0,
          int gonzalez, const double *__restrict__ Ep, int n_el) {
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     // with Ep: S1 = S(v_in) from the element entropy partials first (the sum
     // k_sum_to forms, in the same order)
-    double S1 = Ep ? co_sum_partials(Ep, n_el, 1, 0, sh) : 0.0;
-    double dot = co_sum_partials(red, nred, 2, 0, sh);
-    double n2 = co_sum_partials(red, nred, 2, 1, sh);
+    double v[3] = {Ep ? co_strided_sum(Ep, threadIdx.x, n_el, blockDim.x, 1, 0, 0.0) : 0.0,
+                   co_strided_sum(red, threadIdx.x, nred, blockDim.x, 2, 0, 0.0),
+                   co_strided_sum(red, threadIdx.x, nred, blockDim.x, 2, 1, 0.0)};
+    co_block_sums<3>(v, sh);
+    double S1 = v[0];
+    const double dot = v[1], n2 = v[2];
     if (threadIdx.x == 0) {
         if (Ep) st->S1 = S1;
         else S1 = st->S1;
@@ -130,7 +133,7 @@ k_lb_fused(int N, const double *__restrict__ vmid, const double *__restrict__ w,
            const double *__restrict__ v1, double *__restrict__ r, double *__restrict__ red7,
            double *__restrict__ red2, co_solver_state *st, unsigned *bar, int *err,
            unsigned bar_blocks, int bar_spins) {
-    __shared__ double sh[32];
+    __shared__ double sh[224];
     __shared__ double sol[3];
     const double lam = use_lambda ? st->lambda : 0.0;
     double m[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -153,15 +156,17 @@ k_lb_fused(int N, const double *__restrict__ vmid, const double *__restrict__ w,
         m[5] += wa * g2;
         m[6] += wa * (x * g1 + y * g2);
     }
-    for (int k = 0; k < 7; k++) {
-        double s = co_block_sum(m[k], sh);
-        if (threadIdx.x == 0) red7[blockIdx.x * 8 + k] = s;
-    }
+    co_block_sums<7>(m, sh);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 7; k++) red7[blockIdx.x * 8 + k] = m[k];
     grid_barrier(bar, bar_blocks, err, bar_spins);
     if (threadIdx.x == 0 && *((volatile int *)err)) st->error = CO_ERR_TIMEOUT;
     // every block reduces the partials in the same fixed order
     double tot[7];
-    for (int k = 0; k < 7; k++) tot[k] = co_sum_partials(red7, gridDim.x, 8, k, sh);
+#pragma unroll
+    for (int k = 0; k < 7; k++)
+        tot[k] = co_strided_sum(red7, threadIdx.x, gridDim.x, blockDim.x, 8, k, 0.0);
+    co_block_sums<7>(tot, sh);
     if (threadIdx.x == 0) {
         double M[9] = {tot[0], 0.0, tot[1], 0.0, tot[0], tot[2], tot[1], tot[2], tot[3]};
         double b[3] = {-tot[4], -tot[5], -tot[6]};
@@ -192,11 +197,11 @@ k_lb_fused(int N, const double *__restrict__ vmid, const double *__restrict__ w,
         }
     }
     if (r) {
-        double s1 = co_block_sum(sr, sh);
-        double s2 = co_block_sum(sv, sh);
+        double s[2] = {sr, sv};
+        co_block_sums<2>(s, sh);
         if (threadIdx.x == 0) {
-            red2[blockIdx.x * 2 + 0] = s1;
-            red2[blockIdx.x * 2 + 1] = s2;
+            red2[blockIdx.x * 2 + 0] = s[0];
+            red2[blockIdx.x * 2 + 1] = s[1];
         }
     }
 }
@@ -209,7 +214,7 @@ __global__ void __launch_bounds__(CO_RED_THREADS)
 k_lb_part(int N, const double *__restrict__ vmid, const double *__restrict__ w,
           double *__restrict__ g, const double *__restrict__ dv, int use_lambda,
           const co_solver_state *st, double *__restrict__ red7) {
-    __shared__ double sh[32];
+    __shared__ double sh[224];
     const double lam = use_lambda ? st->lambda : 0.0;
     double m[7] = {0, 0, 0, 0, 0, 0, 0};
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < N; a += gridDim.x * blockDim.x) {
@@ -230,10 +235,9 @@ k_lb_part(int N, const double *__restrict__ vmid, const double *__restrict__ w,
         m[5] += wa * g2;
         m[6] += wa * (x * g1 + y * g2);
     }
-    for (int k = 0; k < 7; k++) {
-        double s = co_block_sum(m[k], sh);
-        if (threadIdx.x == 0) red7[blockIdx.x * 8 + k] = s;
-    }
+    co_block_sums<7>(m, sh);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 7; k++) red7[blockIdx.x * 8 + k] = m[k];
 }
 
 __global__ void __launch_bounds__(CO_RED_THREADS)
@@ -241,10 +245,13 @@ k_lb_apply(int N, int nred7, const double *__restrict__ red7, const double *__re
            const double *__restrict__ g, double nu, double dt, const double *__restrict__ v0,
            double *__restrict__ Gv, const double *__restrict__ v1, double *__restrict__ r,
            double *__restrict__ red2, co_solver_state *st) {
-    __shared__ double sh[32];
+    __shared__ double sh[224];
     __shared__ double sol[3];
     double tot[7];
-    for (int k = 0; k < 7; k++) tot[k] = co_sum_partials(red7, nred7, 8, k, sh);
+#pragma unroll
+    for (int k = 0; k < 7; k++)
+        tot[k] = co_strided_sum(red7, threadIdx.x, nred7, blockDim.x, 8, k, 0.0);
+    co_block_sums<7>(tot, sh);
     if (threadIdx.x == 0) {
         double M[9] = {tot[0], 0.0, tot[1], 0.0, tot[0], tot[2], tot[1], tot[2], tot[3]};
         double b[3] = {-tot[4], -tot[5], -tot[6]};
@@ -275,11 +282,11 @@ k_lb_apply(int N, int nred7, const double *__restrict__ red7, const double *__re
         }
     }
     if (r) {
-        double s1 = co_block_sum(sr, sh);
-        double s2 = co_block_sum(sv, sh);
+        double s[2] = {sr, sv};
+        co_block_sums<2>(s, sh);
         if (threadIdx.x == 0) {
-            red2[blockIdx.x * 2 + 0] = s1;
-            red2[blockIdx.x * 2 + 1] = s2;
+            red2[blockIdx.x * 2 + 0] = s[0];
+            red2[blockIdx.x * 2 + 1] = s[1];
         }
     }
 }
@@ -317,10 +324,12 @@ __global__ void k_state_reset(co_solver_state *st) {
 // (solver.jl:339-391)
 __global__ void __launch_bounds__(256)
 k_ctrl1(const double *__restrict__ red, int nred, co_solver_state *st, co_dev_opts o) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     if (st->done) return;
-    double r2 = co_sum_partials(red, nred, 2, 0, sh);
-    double v2 = co_sum_partials(red, nred, 2, 1, sh);
+    double s2[2] = {co_strided_sum(red, threadIdx.x, nred, blockDim.x, 2, 0, 0.0),
+                    co_strided_sum(red, threadIdx.x, nred, blockDim.x, 2, 1, 0.0)};
+    co_block_sums<2>(s2, sh);
+    const double r2 = s2[0], v2 = s2[1];
     if (threadIdx.x != 0) return;
     if (st->error) {
         st->done = 4;
@@ -1031,10 +1040,12 @@ struct co_defect_dev {
 __global__ void __launch_bounds__(256)
 k_ctrl_outer(const double *__restrict__ red, int nred, co_solver_state *st, co_defect_dev o,
              int stage) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     if (st->done) return;
-    double r2 = co_sum_partials(red, nred, 2, 0, sh);
-    double v2 = co_sum_partials(red, nred, 2, 1, sh);
+    double s2[2] = {co_strided_sum(red, threadIdx.x, nred, blockDim.x, 2, 0, 0.0),
+                    co_strided_sum(red, threadIdx.x, nred, blockDim.x, 2, 1, 0.0)};
+    co_block_sums<2>(s2, sh);
+    const double r2 = s2[0], v2 = s2[1];
     if (threadIdx.x != 0) return;
     if (st->error) {
         st->done = 4;

@@ -426,41 +426,46 @@ k_mass2(const double *__restrict__ Minv2, const double *__restrict__ y0,
 }
 
 // Element quadrature for r-local (mode 0, functions.jl:158-179) or the entropy
-// partial (mode 1, functions.jl:137-155). One thread per (element, Gauss row
-// q1): nq threads per element and 128 / nq elements per block, so the lanes
-// stay busy for any nq. GB300 issues FP64 at 1/64 of the FP32 rate and these
-// kernels are FP64-issue bound, so the tensor-product form is used throughout:
+// partial (mode 1, functions.jl:137-155). GB300 issues FP64 at 1/64 of the FP32 rate
+// and these kernels are FP64-issue bound, so the tensor-product form is used
+// throughout:
 //   g_b(q1)      = sum_a c_ab p1_a(q1)                 (once per row)
 //   f(q1, q2)    = sum_b g_b(q1) p2_b(q2)
 //   H_b(q1)      = sum_q2 h(q1, q2) p2_b(q2),  h = integrand * w_q * |e|
 //   r_ab         = sum_q1 p1_a(q1) H_b(q1)             (rows added in order)
 // about 400 FP64 operations and nq^2 logarithms per element instead of ~30 per
-// Gauss point plus the logarithm. Fixed summation order: deterministic. Two jobs
-// may share a launch (blockIdx.y selects), e.g. r at v_mid and S at v_in.
+// Gauss point plus the logarithm. One thread per Gauss point takes f and the
+// logarithm (most of the work, and a long latency), one per row the sums over it, in
+// the order of q2: with one thread per row for both, the six logarithms of a row
+// followed each other and the smallest meshes ran on a dozen blocks. 256 / nq^2
+// elements per block. Fixed summation order: deterministic. Two jobs may share a
+// launch (blockIdx.y selects), e.g. r at v_mid and S at v_in.
 struct co_elem_job {
     const double *fc;   // spline coefficients (n_dofs)
     int mode;           // 0: r-local -> out[e][9]; 1: entropy partial -> out[e]
     double *out;
 };
 
-#define ELEM_THREADS 128
+#define ELEM_THREADS 256
+static int elem_per_block(int nq) { return ELEM_THREADS / (nq * nq); }
 __global__ void __launch_bounds__(ELEM_THREADS)
 k_elem(co_elem_job j0, co_elem_job j1, int n1, int n2, int nd1, int nq,
        const double *__restrict__ Tq1, const double *__restrict__ Tq2,
        const double *__restrict__ qw, const double *__restrict__ bp1,
        const double *__restrict__ bp2, int logsq) {
-    __shared__ double part[ELEM_THREADS * 9];
+    __shared__ double part[ELEM_THREADS * 9];   // g of a row, then its nine sums
+    __shared__ double val[ELEM_THREADS];        // integrand (mode 0) or f log f of a point
     const co_elem_job jb = blockIdx.y ? j1 : j0;
-    const int mode = jb.mode;
-    const int epb = ELEM_THREADS / nq;
-    const int t = threadIdx.x, el = t / nq, q1 = t - el * nq;
-    const int e = blockIdx.x * epb + el;
-    const int n_el = n1 * n2;
-    if (el < epb && e < n_el) {
-        const int i = e % n1, j = e / n1;
-        const double jac = (bp1[i + 1] - bp1[i]) * (bp2[j + 1] - bp2[j]);
+    const int mode = jb.mode, np = nq * nq;
+    const int epb = ELEM_THREADS / np, n_el = n1 * n2;
+    const int t = threadIdx.x;
+    // row view: element el, row q1
+    const int el = t / nq, q1 = t - el * nq, e = blockIdx.x * epb + el;
+    const bool row = el < epb && e < n_el;
+    const int i = row ? e % n1 : 0, j = row ? e / n1 : 0;
+    double p1[3];
+    if (row) {
         const double *fc = jb.fc;
-        double p1[3], g[3];
 #pragma unroll
         for (int a = 0; a < 3; a++) p1[a] = Tq1[((size_t)i * 3 + a) * nq + q1];
 #pragma unroll
@@ -468,35 +473,47 @@ k_elem(co_elem_job j0, co_elem_job j1, int n1, int n2, int nd1, int nq,
             const double *cr = fc + i + (j + bb) * nd1;
             double v = cr[0] * p1[0];
             v = fma(cr[1], p1[1], v);
-            g[bb] = fma(cr[2], p1[2], v);
+            part[t * 3 + bb] = fma(cr[2], p1[2], v);
         }
+    }
+    __syncthreads();
+    // point view: element pe, point (pq1, pq2)
+    const int pe = t / np, pq = t - pe * np, pq1 = pq / nq, pq2 = pq - pq1 * nq;
+    if (pe < epb && blockIdx.x * epb + pe < n_el) {
+        const int pj = (blockIdx.x * epb + pe) / n1;
+        const double *g = part + (pe * nq + pq1) * 3;
+        const double *T2 = Tq2 + (size_t)pj * 3 * nq + pq2;
+        double f = g[0] * T2[0];
+        f = fma(g[1], T2[nq], f);
+        f = fma(g[2], T2[2 * nq], f);
+        double v;
+        if (mode == 0) {
+            if (logsq)
+                v = f * f > 1e-60 ? (1 + 0.5 * log(f * f)) : 0.0;
+            else
+                v = f > 1e-30 ? (1 + log(f)) : 0.0;
+        } else if (logsq) {
+            v = f * f > 1e-60 ? f * 0.5 * log(f * f) : 0.0;
+        } else {
+            v = f > 1e-30 ? f * log(f) : 0.0;
+        }
+        val[t] = v;
+    }
+    __syncthreads();
+    if (row) {
+        const double jac = (bp1[i + 1] - bp1[i]) * (bp2[j + 1] - bp2[j]);
         const double wq1 = qw[q1];
-        double H0 = 0.0, H1 = 0.0, H2 = 0.0, sv = 0.0;
+        const double *v = val + el * np + q1 * nq;
         const double *T2 = Tq2 + (size_t)j * 3 * nq;
-        for (int q2 = 0; q2 < nq; q2++) {
-            const double p20 = T2[q2], p21 = T2[nq + q2], p22 = T2[2 * nq + q2];
-            double f = g[0] * p20;
-            f = fma(g[1], p21, f);
-            f = fma(g[2], p22, f);
-            const double wj = wq1 * qw[q2] * jac;
-            if (mode == 0) {
-                double integrand;
-                if (logsq)
-                    integrand = f * f > 1e-60 ? (1 + 0.5 * log(f * f)) : 0.0;
-                else
-                    integrand = f > 1e-30 ? (1 + log(f)) : 0.0;
-                const double h = integrand * wj;
-                H0 = fma(h, p20, H0);
-                H1 = fma(h, p21, H1);
-                H2 = fma(h, p22, H2);
-            } else if (logsq) {
-                if (f * f > 1e-60) sv += -(f * 0.5 * log(f * f) * wj);
-            } else if (f > 1e-30) {
-                sv += -(f * log(f) * wj);
-            }
-        }
         double *o = part + (size_t)t * 9;
         if (mode == 0) {
+            double H0 = 0.0, H1 = 0.0, H2 = 0.0;
+            for (int q2 = 0; q2 < nq; q2++) {
+                const double h = v[q2] * (wq1 * qw[q2] * jac);
+                H0 = fma(h, T2[q2], H0);
+                H1 = fma(h, T2[nq + q2], H1);
+                H2 = fma(h, T2[2 * nq + q2], H2);
+            }
 #pragma unroll
             for (int a = 0; a < 3; a++) {
                 o[a] = p1[a] * H0;
@@ -504,6 +521,8 @@ k_elem(co_elem_job j0, co_elem_job j1, int n1, int n2, int nd1, int nq,
                 o[6 + a] = p1[a] * H2;
             }
         } else {
+            double sv = 0.0;
+            for (int q2 = 0; q2 < nq; q2++) sv = fma(-v[q2], wq1 * qw[q2] * jac, sv);
             o[0] = sv;
         }
     }
@@ -638,7 +657,7 @@ k_grad_L(const double *__restrict__ x, int N, const int *__restrict__ cell,
          const double *__restrict__ P1, const double *__restrict__ P2,
          double *__restrict__ G, const double *__restrict__ w, double *__restrict__ dS,
          const double *__restrict__ dv, double *__restrict__ red, co_lambda_job lam) {
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     double pdot = 0.0, pn2 = 0.0;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < N; a += gridDim.x * blockDim.x) {
         int c = cell[a];
@@ -680,11 +699,11 @@ k_grad_L(const double *__restrict__ x, int N, const int *__restrict__ cell,
         }
     }
     if (red) {
-        double s = co_block_sum(pdot, sh);
-        double n = co_block_sum(pn2, sh);
+        double v[2] = {pdot, pn2};
+        co_block_sums<2>(v, sh);
         if (threadIdx.x == 0) {
-            red[blockIdx.x * 2 + 0] = s;
-            red[blockIdx.x * 2 + 1] = n;
+            red[blockIdx.x * 2 + 0] = v[0];
+            red[blockIdx.x * 2 + 1] = v[1];
         }
         if (lam.st) {
             // the last block to finish forms the Gonzalez lambda (landau_geff!,
@@ -700,13 +719,13 @@ k_grad_L(const double *__restrict__ x, int N, const int *__restrict__ cell,
             __threadfence();
             if (threadIdx.x == 0) *lam.ticket = 0u;
             const int nb = gridDim.x;
-            double S1 = lam.Ep ? co_block_sum(co_strided_sum(lam.Ep, threadIdx.x, lam.n_el,
-                                                             blockDim.x, 1, 0, 0.0), sh)
-                               : 0.0;
-            double dot = co_block_sum(co_strided_sum_cg(red, threadIdx.x, nb, blockDim.x, 2, 0,
-                                                        0.0), sh);
-            double nn = co_block_sum(co_strided_sum_cg(red, threadIdx.x, nb, blockDim.x, 2, 1,
-                                                       0.0), sh);
+            double q[3] = {lam.Ep ? co_strided_sum(lam.Ep, threadIdx.x, lam.n_el, blockDim.x, 1, 0, 0.0)
+                                  : 0.0,
+                           co_strided_sum_cg(red, threadIdx.x, nb, blockDim.x, 2, 0, 0.0),
+                           co_strided_sum_cg(red, threadIdx.x, nb, blockDim.x, 2, 1, 0.0)};
+            co_block_sums<3>(q, sh);
+            double S1 = q[0];
+            const double dot = q[1], nn = q[2];
             if (threadIdx.x == 0) {
                 if (lam.Ep) lam.st->S1 = S1;
                 else S1 = lam.st->S1;
@@ -727,7 +746,7 @@ k_loggrad(const double *__restrict__ x, int N, const int *__restrict__ cell,
           const double *__restrict__ C1, const double *__restrict__ C2,
           double *__restrict__ g, const double *__restrict__ w,
           const double *__restrict__ dv, double *__restrict__ red) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     double pdot = 0.0, pn2 = 0.0;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < N; a += gridDim.x * blockDim.x) {
         int c = cell[a];
@@ -764,11 +783,11 @@ k_loggrad(const double *__restrict__ x, int N, const int *__restrict__ cell,
         }
     }
     if (red) {
-        double s = co_block_sum(pdot, sh);
-        double n = co_block_sum(pn2, sh);
+        double v[2] = {pdot, pn2};
+        co_block_sums<2>(v, sh);
         if (threadIdx.x == 0) {
-            red[blockIdx.x * 2 + 0] = s;
-            red[blockIdx.x * 2 + 1] = n;
+            red[blockIdx.x * 2 + 0] = v[0];
+            red[blockIdx.x * 2 + 1] = v[1];
         }
     }
 }
@@ -1027,7 +1046,7 @@ int co_project_sorted(co_ctx *c, double *f_out) { return co_project_two(c, f_out
 int co_r_and_entropy_dev(co_ctx *c, const double *f, double *r, const double *fS) {
     co_elem_job jr = {f, 0, c->E};
     co_elem_job js = {fS, 1, c->Ep};
-    k_elem<<<dim3(co_cdiv(c->n_el, ELEM_THREADS / c->nq), fS ? 2 : 1), ELEM_THREADS, 0,
+    k_elem<<<dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), fS ? 2 : 1), ELEM_THREADS, 0,
              c->stream>>>(jr, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1,
                           c->bp2, (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     k_dofgather<<<dim3(co_cdiv(c->n_dofs, 128), 1), 128, 0, c->stream>>>(
@@ -1040,7 +1059,7 @@ int co_r_and_entropy_dev(co_ctx *c, const double *f, double *r, const double *fS
 int co_r_solve_dev(co_ctx *c, const double *f, double *L, const double *fS) {
     co_elem_job jr = {f, 0, c->E};
     co_elem_job js = {fS, 1, c->Ep};
-    k_elem<<<dim3(co_cdiv(c->n_el, ELEM_THREADS / c->nq), fS ? 2 : 1), ELEM_THREADS, 0,
+    k_elem<<<dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), fS ? 2 : 1), ELEM_THREADS, 0,
              c->stream>>>(jr, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1,
                           c->bp2, (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     c->launches++;
@@ -1054,7 +1073,7 @@ int co_compute_r_dev(co_ctx *c, const double *f, double *r) {
 
 int co_entropy_parts_dev(co_ctx *c, const double *f) {
     co_elem_job js = {f, 1, c->Ep};
-    k_elem<<<dim3(co_cdiv(c->n_el, ELEM_THREADS / c->nq), 1), ELEM_THREADS, 0, c->stream>>>(
+    k_elem<<<dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), 1), ELEM_THREADS, 0, c->stream>>>(
         js, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
         (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     c->launches++;
