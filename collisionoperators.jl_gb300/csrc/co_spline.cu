@@ -83,7 +83,7 @@ struct co_locate_job {
 // one or two marker sets (blockIdx.y). The reference coordinate is (v - bp[i])
 // times the cell's reciprocal width (within one ulp of the quotient; an FP64
 // division costs ~10 FP64 issue slots on this GPU).
-__global__ void __launch_bounds__(CO_CHUNK)
+__global__ void __launch_bounds__(CO_CHUNK)   // one sort chunk per block (sort_chunk)
 k_locate_hist(co_locate_job j0, co_locate_job j1, int N, const double *__restrict__ bp1,
               int n1, const double *__restrict__ bp2, int n2, const double *__restrict__ ih1,
               const double *__restrict__ ih2, int n_el) {
@@ -91,7 +91,7 @@ k_locate_hist(co_locate_job j0, co_locate_job j1, int N, const double *__restric
     const co_locate_job J = blockIdx.y ? j1 : j0;
     for (int i = threadIdx.x; i < n_el; i += blockDim.x) hs[i] = 0;
     __syncthreads();
-    int a = blockIdx.x * CO_CHUNK + threadIdx.x;
+    int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a < N) {
         double v1 = J.x[a], v2 = J.x[N + a];
         if (J.v0) {
@@ -135,14 +135,14 @@ k_cellcount(co_sortset s0, co_sortset s1, int nchunk, int n_el, unsigned *ticket
         const int *__restrict__ hist = S.hist;
         int *__restrict__ hoff = S.hoff;
         int run = 0, k = 0;
-        // eight chunk counts loaded ahead of the running sum: one L2 round trip
-        // per eight chunks instead of per chunk
-        for (; k + 8 <= nchunk; k += 8) {
-            int h[8];
+        // sixteen chunk counts loaded ahead of the running sum: one L2 round trip
+        // per sixteen chunks instead of per chunk
+        for (; k + 16 <= nchunk; k += 16) {
+            int h[16];
 #pragma unroll
-            for (int u = 0; u < 8; u++) h[u] = hist[(size_t)(k + u) * n_el + c];
+            for (int u = 0; u < 16; u++) h[u] = hist[(size_t)(k + u) * n_el + c];
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
+            for (int u = 0; u < 16; u++) {
                 hoff[(size_t)(k + u) * n_el + c] = run;
                 run += h[u];
             }
@@ -197,14 +197,14 @@ k_perm(co_sortset s0, co_sortset s1, int N, int n_el, int n1, const double *__re
     const co_sortset S = blockIdx.y ? s1 : s0;
     for (int i = threadIdx.x; i < n_el; i += blockDim.x) run[i] = 0;
     __syncthreads();
-    int a = blockIdx.x * CO_CHUNK + threadIdx.x;
+    int a = blockIdx.x * blockDim.x + threadIdx.x;
     int c = a < N ? S.cell[a] : -2;
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned peers = __match_any_sync(0xffffffffu, c);
     int rank = __popc(peers & ((1u << lane) - 1u));
     int leader = __ffs(peers) - 1;
     int base = 0;
-    for (int wv = 0; wv < (CO_CHUNK >> 5); wv++) {
+    for (int wv = 0; wv < (int)(blockDim.x >> 5); wv++) {
         if (warp == wv) {
             int b = 0;
             if (c >= 0 && lane == leader) {
@@ -955,16 +955,27 @@ static int ensure_gs(co_ctx *c) {
     return CO_OK;
 }
 
+// Markers of a sort chunk (one block of the locate and placement kernels). Up to
+// 16,384 markers chunks of 256: four times the blocks, and 8 instead of 32 warp turns
+// in the placement; the per-chunk histograms stay at 64 rows, which k_cellcount walks
+// in order, so larger sets keep 1,024. The sorted order does not depend on it.
+static int sort_chunk(int N) { return N <= 64 * 256 ? 256 : CO_CHUNK; }
+static size_t sort_rows(int cap) {   // histogram rows for any N <= cap
+    const int a = co_cdiv(cap, CO_CHUNK), b = co_cdiv(cap < 64 * 256 ? cap : 64 * 256, 256);
+    return a > b ? a : b;
+}
+
 // locate + stable sort of one or two marker sets (jobs j0 -> set 0, j1 -> set 1)
 static int sort_sets(co_ctx *c, const co_locate_job &j0, const co_locate_job &j1, int nsets,
                      int N) {
     co_bufs &b = c->mb;
     const co_sortset s0 = primary_set(c), s1 = nsets > 1 ? c->gs : s0;
-    int nchunk = co_cdiv(N, CO_CHUNK);
+    const int chunk = sort_chunk(N);
+    int nchunk = co_cdiv(N, chunk);
     if (nchunk == 0) nchunk = 1;
     size_t sm = sizeof(int) * (size_t)c->n_el;
     if (N > 0) {
-        k_locate_hist<<<dim3(nchunk, nsets), CO_CHUNK, sm, c->stream>>>(
+        k_locate_hist<<<dim3(nchunk, nsets), chunk, sm, c->stream>>>(
             j0, j1, N, c->bp1, c->n1, c->bp2, c->n2, c->ih1, c->ih2, c->n_el);
         c->launches++;
     } else {
@@ -975,7 +986,7 @@ static int sort_sets(co_ctx *c, const co_locate_job &j0, const co_locate_job &j1
         s0, s1, N > 0 ? nchunk : 1, c->n_el, c->tickets);
     c->launches++;
     if (N > 0) {
-        k_perm<<<dim3(nchunk, nsets), CO_CHUNK, sm, c->stream>>>(s0, s1, N, c->n_el, c->n1,
+        k_perm<<<dim3(nchunk, nsets), chunk, sm, c->stream>>>(s0, s1, N, c->n_el, c->n1,
                                                                  b.w, c->P1, c->P2);
         c->launches++;
     }
@@ -1204,7 +1215,7 @@ int co_ensure_capacity(co_ctx *c, int N, int m) {
         if ((rc = grow(&b.gwmax, (size_t)cap / 256))) return rc;
         if ((rc = grow(&b.pdot, n2))) return rc;
         if ((rc = grow(&b.pA, 3 * (size_t)cap))) return rc;
-        int nchunk = co_cdiv(cap, CO_CHUNK);
+        const int nchunk = (int)sort_rows(cap);
         if ((rc = grow(&b.hist, (size_t)nchunk * c->n_el))) return rc;
         if ((rc = grow(&b.hoff, (size_t)nchunk * c->n_el))) return rc;
         b.nchunk_cap = nchunk;
