@@ -178,7 +178,7 @@ static void free_ctx(co_ctx *c) {
                     c->mb.Gp, c->mb.vbest, c->mb.v1, c->mb.v0, c->mb.w, c->mb.vin, c->mb.dotv,
                     c->mb.cell, c->mb.inv, c->mb.xi, c->mb.perm, c->mb.scell, c->mb.sw,
                     c->mb.sphi, c->mb.px, c->mb.pg, c->mb.pw, c->mb.pf_x, c->mb.pf_g, c->mb.pf_w, c->mb.pf_wl,
-                    c->mb.fx_x, c->mb.fx_w, c->mb.fx_g, c->mb.pwn, c->mb.unit, c->mb.gwmax,
+                    c->mb.fx_x,
                     c->mb.pdot, c->mb.pA, c->mb.part, c->mb.hist, c->mb.hoff, c->mb.count,
                     c->mb.cstart, c->mb.red, c->mb.dF, c->mb.dG, c->mb.Gk, c->mb.Phi,
                     c->mb.Adef, c->mb.aa, c->mb.pc, c->st2, c->st3, c->tickets};
