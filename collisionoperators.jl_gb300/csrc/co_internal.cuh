@@ -148,6 +148,7 @@ struct co_ctx {
     co_solver_state *st2;    // inner-solve state of the defect correction
     co_solver_state *st3;    // outer Anderson window of the defect correction
     co_solver_state *st_host;  // pinned mirror
+    int *bad_host;             // pinned: an argument was not finite (load_finite)
     double *hstage;          // pinned host staging (grows)
     size_t hstage_cap;
     int pair_split_fp64, pair_split_fp32;  // split factors of the plain kernels (0 = auto)
