@@ -154,6 +154,7 @@ struct co_ctx {
     int pair_split_fp64, pair_split_fp32;  // split factors of the plain kernels (0 = auto)
     int pair_symmetric;      // 1: Newton's-third-law kernels (default), 0: one-sided
     int nsm;
+    int early;                 // co_launch: grids start before the one before them ends
     int fixed_ex;            // exponent of the fixed-point pair sum's coordinate scale
     // launch counter (kernels of this library launched through the context)
     unsigned long long launches;
@@ -170,6 +171,39 @@ struct co_ctx {
     struct co_step_bufs *sb;  // buffers of co_step_learned (co_step.cu), allocated on first use
     struct co_nk_bufs *nk;    // buffers of the Newton-Krylov solve (co_newton.cu), on first use
 };
+
+// First statement of the kernels that co_launch launches: a grid may start while the one
+// before it in the stream still runs, waits here until that grid is done and its writes
+// are visible, and lets the next grid start in turn. Each of these kernels waits, so all
+// grids before it are done as well.
+__device__ __forceinline__ void co_grid_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
+// Launches of the O(N) chain, each a few us long: starting a grid early takes its launch
+// out of the gap between two of them (2,048 markers: projection 64 -> 53 us, Landau map
+// 178 -> 155). Up to CO_EARLY_MAX markers: above, the blocks of a grid that started early
+// crowd the SMs the grid before left free, and the longer stages lose more than the gap
+// (Lenard-Bernstein map of 16,384 markers 181 -> 172 us, of 25,000 196 -> 198, of 50,000
+// 233 -> 245). Not in a captured graph, whose launches have no such gap.
+#define CO_EARLY_MAX 20000
+template <typename... P, typename... A>
+static void co_launch(co_ctx *c, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... a) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cfg.attrs = &at;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cfg.numAttrs = c->early && cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess &&
+                   cap == cudaStreamCaptureStatusNone;
+    cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+}
 
 // ------------------------------------------------------------- helpers
 #define CO_CK(call)                                                   \

@@ -1191,6 +1191,7 @@ k_pack_landau(const int *__restrict__ perm, const int *__restrict__ Mp, int Mpad
               const double *__restrict__ vmid, const double *__restrict__ dS,
               const double *__restrict__ dv, const double *__restrict__ w,
               const co_solver_state *__restrict__ st, int use_lambda, int mode, co_pack_out o) {
+    co_grid_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = p < *Mp;
     double x1 = 0.0, x2 = 0.0, G1 = 0.0, G2 = 0.0, wa = 0.0;
@@ -1213,6 +1214,7 @@ __global__ void __launch_bounds__(256)
 k_pack_plain(const int *__restrict__ perm, const int *__restrict__ Mp, int Mpad, int N,
              const double *__restrict__ v, const double *__restrict__ G,
              const double *__restrict__ w, int mode, co_pack_out o) {
+    co_grid_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = p < *Mp;
     double x1 = 0.0, x2 = 0.0, G1 = 0.0, G2 = 0.0, wa = 0.0;
@@ -1236,6 +1238,7 @@ k_unpack_update(const int *__restrict__ inv, int N, const double *__restrict__ p
                 double dt, const double *__restrict__ v0, double *__restrict__ Gv,
                 double *__restrict__ dotv, const double *__restrict__ v1, double *__restrict__ r,
                 double *__restrict__ red) {
+    co_grid_wait();
     __shared__ double sh[64];
     double sr = 0.0, sv = 0.0;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < N; a += gridDim.x * blockDim.x) {
@@ -1432,8 +1435,8 @@ int co_pack_plain(co_ctx *c, int N, int Mub, int precision, const double *x, con
     const int *Mp = c->mb.cstart + c->n_el;
     co_bufs &b = c->mb;
     int Mpad = co_cdiv(Mub, 256) * 256;  // whole tiles of up to 256 markers
-    k_pack_plain<<<Mpad / 256, 256, 0, c->stream>>>(b.perm, Mp, Mpad, N, x, G, b.w,
-                                                    co_pack_mode(precision), pack_out(c));
+    co_launch(c, k_pack_plain, Mpad / 256, 256, 0, b.perm, Mp, Mpad, N, x, G, b.w,
+              co_pack_mode(precision), pack_out(c));
     c->launches++;
     CO_CK(cudaGetLastError());
     return co_use_fixed(c, Mub, precision) ? co_pair_fixed_pack(c, Mub, Mpad / 256) : CO_OK;
@@ -1444,9 +1447,8 @@ int co_pack_landau(co_ctx *c, int N, int Mub, int precision, int gonzalez) {
     const int *Mp = c->mb.cstart + c->n_el;
     co_bufs &b = c->mb;
     int Mpad = co_cdiv(Mub, 256) * 256;  // whole tiles of up to 256 markers
-    k_pack_landau<<<Mpad / 256, 256, 0, c->stream>>>(b.perm, Mp, Mpad, N, b.vmid, b.dS, b.dv, b.w,
-                                                     c->st, gonzalez, co_pack_mode(precision),
-                                                     pack_out(c));
+    co_launch(c, k_pack_landau, Mpad / 256, 256, 0, b.perm, Mp, Mpad, N, b.vmid, b.dS, b.dv, b.w,
+              c->st, gonzalez, co_pack_mode(precision), pack_out(c));
     c->launches++;
     CO_CK(cudaGetLastError());
     return co_use_fixed(c, Mub, precision) ? co_pair_fixed_pack(c, Mub, Mpad / 256) : CO_OK;
@@ -1457,9 +1459,8 @@ int co_unpack_update(co_ctx *c, int N, double dt, double *Gv, const double *v0,
     if (N == 0) return CO_OK;
     int g = co_cdiv(N, CO_RED_THREADS);
     if (g > c->mb.red_cap) g = c->mb.red_cap;
-    k_unpack_update<<<g, CO_RED_THREADS, 0, c->stream>>>(c->mb.inv, N, c->mb.pdot,
-                                                         (size_t)c->mb.cap, dt, v0, Gv,
-                                                         c->mb.dotv, v1, r, red);
+    co_launch(c, k_unpack_update, g, CO_RED_THREADS, 0, c->mb.inv, N, c->mb.pdot,
+              (size_t)c->mb.cap, dt, v0, Gv, c->mb.dotv, v1, r, red);
     c->launches++;
     CO_CK(cudaGetLastError());
     return CO_OK;

@@ -256,6 +256,7 @@ template <int W, int NC>
 __global__ void __launch_bounds__(32 * W)
 k_pair_fixed_sym(const co_fixed_ops o, int nt, int H, int KC, double *__restrict__ gpart,
                  double *__restrict__ apart) {
+    co_grid_wait();
     __shared__ fixed_smem<W, NC> sm;
     const int I = blockIdx.x % nt, chunk = blockIdx.x / nt;
     const int k0 = chunk * KC, k1 = min(H + 1, k0 + KC);
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(32 * FIXED_SL)
 k_fixed_reduce(const double *__restrict__ gpart, const double *__restrict__ apart, int nt, int H,
                int nchunk, int TS, const double *__restrict__ unit, double *__restrict__ pdot,
                double *__restrict__ pA, size_t ld) {
+    co_grid_wait();
     __shared__ double sh[NC][FIXED_SL][33];
     const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const int p = blockIdx.x * 32 + lane;          // TS is a multiple of 32
@@ -328,6 +330,7 @@ k_pair_fixed_pack(const double2 *__restrict__ px, const double2 *__restrict__ pg
                   const double2 *__restrict__ part, int npart, int ex, double c1, double c2,
                   longlong2 *__restrict__ ox, int4 *__restrict__ og, fx64 *__restrict__ ow,
                   double *__restrict__ pwn, double *__restrict__ unit) {
+    co_grid_wait();
     __shared__ double shg[8], shw[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double gm = 0.0, wm = 0.0;
@@ -398,9 +401,8 @@ int co_pair_fixed_pack(co_ctx *c, int Mub, int npart) {
     const int ex = ilogb(big) + 2;
     c->fixed_ex = ex;
     const int Mpad = co_cdiv(Mub, 256) * 256;
-    k_pair_fixed_pack<<<Mpad / 256, 256, 0, c->stream>>>(
-        b.px, b.pg, b.pw, b.cstart + c->n_el, Mpad, b.gwmax, npart, ex, c1, c2,
-        (longlong2 *)b.fx_x, b.fx_g, b.fx_w, b.pwn, b.unit);
+    co_launch(c, k_pair_fixed_pack, Mpad / 256, 256, 0, b.px, b.pg, b.pw, b.cstart + c->n_el, Mpad,
+              b.gwmax, npart, ex, c1, c2, (longlong2 *)b.fx_x, b.fx_g, b.fx_w, b.pwn, b.unit);
     c->launches++;
     CO_CK(cudaGetLastError());
     return CO_OK;
@@ -447,11 +449,11 @@ static int fixed_run(co_ctx *c, int Mub, int KC, int prof_kind) {
     if (rc) return rc;
     double *gpart = c->mb.part, *apart = c->mb.part + gsz;
     co_prof_begin(c, prof_kind);
-    k_pair_fixed_sym<W, NC><<<nt * nchunk, TS, 0, c->stream>>>(co_fixed_operands(c), nt, H, KC,
-                                                               gpart, apart);
+    co_launch(c, k_pair_fixed_sym<W, NC>, nt * nchunk, TS, 0, co_fixed_operands(c), nt, H, KC,
+              gpart, apart);
     co_prof_end(c);
-    k_fixed_reduce<NC><<<nt * W, 32 * FIXED_SL, 0, c->stream>>>(
-        gpart, apart, nt, H, nchunk, TS, c->mb.unit, c->mb.pdot, c->mb.pA, (size_t)c->mb.cap);
+    co_launch(c, k_fixed_reduce<NC>, nt * W, 32 * FIXED_SL, 0, gpart, apart, nt, H, nchunk, TS,
+              c->mb.unit, c->mb.pdot, c->mb.pA, (size_t)c->mb.cap);
     c->launches += 2;
     CO_CK(cudaGetLastError());
     return CO_OK;

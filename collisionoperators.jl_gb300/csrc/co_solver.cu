@@ -55,6 +55,7 @@ static const char *prec_name(int p) {
 __global__ void __launch_bounds__(256)
 k_lambda(const double *__restrict__ red, int nred, co_solver_state *st, double S0,
          int gonzalez, const double *__restrict__ Ep, int n_el) {
+    co_grid_wait();
     __shared__ double sh[96];
     // with Ep: S1 = S(v_in) from the element entropy partials first (the sum
     // k_sum_to forms, in the same order)
@@ -690,8 +691,8 @@ static int landau_tail(co_ctx *c, int gonzalez, int N, double S0, int nred) {
     if (N > 0)
         return co_grad_L_lambda_dev(c, b.vmid, N, c->L, b.G, b.w, b.dS, b.dv, b.red, S0,
                                     gonzalez, gonzalez ? c->Ep : nullptr);
-    k_lambda<<<1, 256, 0, c->stream>>>(b.red, 0, c->st, S0, gonzalez,
-                                       gonzalez ? c->Ep : nullptr, c->n_el);
+    co_launch(c, k_lambda, 1, 256, 0, b.red, 0, c->st, S0, gonzalez, gonzalez ? c->Ep : nullptr,
+              c->n_el);
     c->launches++;
     (void)nred;
     CO_CK(cudaGetLastError());
@@ -726,8 +727,8 @@ static int picard_map_impl(co_ctx *c, int model, int gonzalez, double nu, int pr
     if (model == CO_MODEL_LB) {
         if (gonzalez && (rc = co_entropy_parts_dev(c, c->fin))) return rc;
         if ((rc = co_loggrad_dev(c, b.vmid, N, c->f, b.G, b.w, b.dv, b.red))) return rc;
-        k_lambda<<<1, 256, 0, c->stream>>>(b.red, nred, c->st, S0, gonzalez,
-                                           gonzalez ? c->Ep : nullptr, c->n_el);
+        co_launch(c, k_lambda, 1, 256, 0, b.red, nred, c->st, S0, gonzalez,
+                  gonzalez ? c->Ep : nullptr, c->n_el);
         c->launches++;
         CO_CK(cudaGetLastError());
         if (c->lb_two_pass) {

@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(CO_CHUNK)   // one sort chunk per block (sort_
 k_locate_hist(co_locate_job j0, co_locate_job j1, int N, const double *__restrict__ bp1,
               int n1, const double *__restrict__ bp2, int n2, const double *__restrict__ ih1,
               const double *__restrict__ ih2, int n_el) {
+    co_grid_wait();
     extern __shared__ int hs[];
     const co_locate_job J = blockIdx.y ? j1 : j0;
     for (int i = threadIdx.x; i < n_el; i += blockDim.x) hs[i] = 0;
@@ -129,6 +130,7 @@ k_locate_hist(co_locate_job j0, co_locate_job j1, int N, const double *__restric
 // cell starts of the sorted order). Integer sums: exact, whatever the order.
 __global__ void __launch_bounds__(256)
 k_cellcount(co_sortset s0, co_sortset s1, int nchunk, int n_el, unsigned *tickets) {
+    co_grid_wait();
     const co_sortset S = blockIdx.y ? s1 : s0;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < n_el) {
@@ -193,6 +195,7 @@ k_cellcount(co_sortset s0, co_sortset s1, int nchunk, int n_el, unsigned *ticket
 __global__ void __launch_bounds__(CO_CHUNK)
 k_perm(co_sortset s0, co_sortset s1, int N, int n_el, int n1, const double *__restrict__ w,
        const double *__restrict__ P1, const double *__restrict__ P2) {
+    co_grid_wait();
     extern __shared__ int run[];
     const co_sortset S = blockIdx.y ? s1 : s0;
     for (int i = threadIdx.x; i < n_el; i += blockDim.x) run[i] = 0;
@@ -240,6 +243,7 @@ k_perm(co_sortset s0, co_sortset s1, int N, int n_el, int n1, const double *__re
 // Deterministic run to run.
 __global__ void __launch_bounds__(128)
 k_cellsum(co_sortset s0, co_sortset s1, int n_el) {
+    co_grid_wait();
     __shared__ double part[4][9];
     const co_sortset S = blockIdx.y ? s1 : s0;
     const int c = blockIdx.x;
@@ -329,6 +333,7 @@ __global__ void __launch_bounds__(256)
 k_mass1(const double *__restrict__ Minv1, const double *__restrict__ b0,
         double *__restrict__ y0, const double *__restrict__ b1, double *__restrict__ y1,
         int nd1, int nd2) {
+    co_grid_wait();
     const double *__restrict__ b = blockIdx.y ? b1 : b0;
     double *__restrict__ y = blockIdx.y ? y1 : y0;
     const int ng1 = (nd1 + MASS_OUT - 1) / MASS_OUT;
@@ -361,6 +366,7 @@ __global__ void __launch_bounds__(256)
 k_gather_mass1(const double *__restrict__ src0, double *__restrict__ y0,
                const double *__restrict__ src1, double *__restrict__ y1,
                const double *__restrict__ Minv1, int n1, int n2, int nd1, int nd2) {
+    co_grid_wait();
     extern __shared__ double col[];
     const double *__restrict__ src = blockIdx.y ? src1 : src0;
     double *__restrict__ y = blockIdx.y ? y1 : y0;
@@ -404,6 +410,7 @@ __global__ void __launch_bounds__(256)
 k_mass2(const double *__restrict__ Minv2, const double *__restrict__ y0,
         double *__restrict__ out0, const double *__restrict__ y1, double *__restrict__ out1,
         int nd1, int nd2) {
+    co_grid_wait();
     const double *__restrict__ y = blockIdx.y ? y1 : y0;
     double *__restrict__ out = blockIdx.y ? out1 : out0;
     const int ng1 = (nd1 + MASS_OUT - 1) / MASS_OUT;
@@ -453,6 +460,7 @@ k_elem(co_elem_job j0, co_elem_job j1, int n1, int n2, int nd1, int nq,
        const double *__restrict__ Tq1, const double *__restrict__ Tq2,
        const double *__restrict__ qw, const double *__restrict__ bp1,
        const double *__restrict__ bp2, int logsq) {
+    co_grid_wait();
     __shared__ double part[ELEM_THREADS * 9];   // g of a row, then its nine sums
     __shared__ double val[ELEM_THREADS];        // integrand (mode 0) or f log f of a point
     const co_elem_job jb = blockIdx.y ? j1 : j0;
@@ -657,6 +665,7 @@ k_grad_L(const double *__restrict__ x, int N, const int *__restrict__ cell,
          const double *__restrict__ P1, const double *__restrict__ P2,
          double *__restrict__ G, const double *__restrict__ w, double *__restrict__ dS,
          const double *__restrict__ dv, double *__restrict__ red, co_lambda_job lam) {
+    co_grid_wait();
     __shared__ double sh[96];
     double pdot = 0.0, pn2 = 0.0;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < N; a += gridDim.x * blockDim.x) {
@@ -746,6 +755,7 @@ k_loggrad(const double *__restrict__ x, int N, const int *__restrict__ cell,
           const double *__restrict__ C1, const double *__restrict__ C2,
           double *__restrict__ g, const double *__restrict__ w,
           const double *__restrict__ dv, double *__restrict__ red) {
+    co_grid_wait();
     __shared__ double sh[64];
     double pdot = 0.0, pn2 = 0.0;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < N; a += gridDim.x * blockDim.x) {
@@ -971,23 +981,24 @@ static int sort_sets(co_ctx *c, const co_locate_job &j0, const co_locate_job &j1
     co_bufs &b = c->mb;
     const co_sortset s0 = primary_set(c), s1 = nsets > 1 ? c->gs : s0;
     const int chunk = sort_chunk(N);
+    c->early = N <= CO_EARLY_MAX;
     int nchunk = co_cdiv(N, chunk);
     if (nchunk == 0) nchunk = 1;
     size_t sm = sizeof(int) * (size_t)c->n_el;
     if (N > 0) {
-        k_locate_hist<<<dim3(nchunk, nsets), chunk, sm, c->stream>>>(
-            j0, j1, N, c->bp1, c->n1, c->bp2, c->n2, c->ih1, c->ih2, c->n_el);
+        co_launch(c, k_locate_hist, dim3(nchunk, nsets), chunk, sm, j0, j1, N, c->bp1, c->n1,
+                  c->bp2, c->n2, c->ih1, c->ih2, c->n_el);
         c->launches++;
     } else {
         CO_CK(cudaMemsetAsync(s0.hist, 0, sizeof(int) * c->n_el, c->stream));
         if (nsets > 1) CO_CK(cudaMemsetAsync(s1.hist, 0, sizeof(int) * c->n_el, c->stream));
     }
-    k_cellcount<<<dim3(co_cdiv(c->n_el, 256), nsets), 256, 0, c->stream>>>(
-        s0, s1, N > 0 ? nchunk : 1, c->n_el, c->tickets);
+    co_launch(c, k_cellcount, dim3(co_cdiv(c->n_el, 256), nsets), 256, 0, s0, s1,
+              N > 0 ? nchunk : 1, c->n_el, c->tickets);
     c->launches++;
     if (N > 0) {
-        k_perm<<<dim3(nchunk, nsets), chunk, sm, c->stream>>>(s0, s1, N, c->n_el, c->n1,
-                                                                 b.w, c->P1, c->P2);
+        co_launch(c, k_perm, dim3(nchunk, nsets), chunk, sm, s0, s1, N, c->n_el, c->n1, b.w, c->P1,
+                  c->P2);
         c->launches++;
     }
     CO_CK(cudaGetLastError());
@@ -1016,10 +1027,10 @@ static int mass_solve_two(co_ctx *c, const double *r0, double *y0, double *o0,
                           const double *r1, double *y1, double *o1, int nsets) {
     // one warp per MASS_OUT outputs of a column, eight warps per block
     const int nw = co_cdiv(c->nd1, MASS_OUT) * c->nd2;
-    k_mass1<<<dim3(co_cdiv(nw, 8), nsets), 256, 0, c->stream>>>(c->Minv1, r0, y0, r1, y1,
-                                                                 c->nd1, c->nd2);
-    k_mass2<<<dim3(co_cdiv(nw, 8), nsets), 256, 0, c->stream>>>(c->Minv2, y0, o0, y1, o1,
-                                                                 c->nd1, c->nd2);
+    co_launch(c, k_mass1, dim3(co_cdiv(nw, 8), nsets), 256, 0, c->Minv1, r0, y0, r1, y1, c->nd1,
+              c->nd2);
+    co_launch(c, k_mass2, dim3(co_cdiv(nw, 8), nsets), 256, 0, c->Minv2, y0, o0, y1, o1, c->nd1,
+              c->nd2);
     c->launches += 2;
     CO_CK(cudaGetLastError());
     return CO_OK;
@@ -1032,11 +1043,11 @@ int co_mass_solve_dev(co_ctx *c, const double *rhs, double *out) {
 // cell sums -> (dof gather + M1^{-1}) -> M2^{-1}, for one or two marker sets
 static int gather_solve_two(co_ctx *c, const double *e0, double *y0, double *o0,
                             const double *e1, double *y1, double *o1, int nsets) {
-    k_gather_mass1<<<dim3(c->nd2, nsets), 256, sizeof(double) * c->nd1, c->stream>>>(
-        e0, y0, e1, y1, c->Minv1, c->n1, c->n2, c->nd1, c->nd2);
+    co_launch(c, k_gather_mass1, dim3(c->nd2, nsets), 256, sizeof(double) * c->nd1, e0, y0, e1, y1,
+              c->Minv1, c->n1, c->n2, c->nd1, c->nd2);
     const int nw = co_cdiv(c->nd1, MASS_OUT) * c->nd2;
-    k_mass2<<<dim3(co_cdiv(nw, 8), nsets), 256, 0, c->stream>>>(c->Minv2, y0, o0, y1, o1,
-                                                                 c->nd1, c->nd2);
+    co_launch(c, k_mass2, dim3(co_cdiv(nw, 8), nsets), 256, 0, c->Minv2, y0, o0, y1, o1, c->nd1,
+              c->nd2);
     c->launches += 2;
     CO_CK(cudaGetLastError());
     return CO_OK;
@@ -1045,7 +1056,7 @@ static int gather_solve_two(co_ctx *c, const double *e0, double *y0, double *o0,
 int co_project_two(co_ctx *c, double *f0, double *f1, int two) {
     const int nsets = two ? 2 : 1;
     const co_sortset s0 = primary_set(c), s1 = two ? c->gs : s0;
-    k_cellsum<<<dim3(c->n_el, nsets), 128, 0, c->stream>>>(s0, s1, c->n_el);
+    co_launch(c, k_cellsum, dim3(c->n_el, nsets), 128, 0, s0, s1, c->n_el);
     c->launches++;
     CO_CK(cudaGetLastError());
     return gather_solve_two(c, s0.bS, s0.y, f0, s1.bS, s1.y, two ? f1 : f0, nsets);
@@ -1057,9 +1068,9 @@ int co_project_sorted(co_ctx *c, double *f_out) { return co_project_two(c, f_out
 int co_r_and_entropy_dev(co_ctx *c, const double *f, double *r, const double *fS) {
     co_elem_job jr = {f, 0, c->E};
     co_elem_job js = {fS, 1, c->Ep};
-    k_elem<<<dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), fS ? 2 : 1), ELEM_THREADS, 0,
-             c->stream>>>(jr, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1,
-                          c->bp2, (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
+    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), fS ? 2 : 1), ELEM_THREADS,
+              0, jr, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
+              (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     k_dofgather<<<dim3(co_cdiv(c->n_dofs, 128), 1), 128, 0, c->stream>>>(
         c->E, r, c->E, r, c->n1, c->n2, c->nd1, c->nd2);
     c->launches += 2;
@@ -1070,9 +1081,9 @@ int co_r_and_entropy_dev(co_ctx *c, const double *f, double *r, const double *fS
 int co_r_solve_dev(co_ctx *c, const double *f, double *L, const double *fS) {
     co_elem_job jr = {f, 0, c->E};
     co_elem_job js = {fS, 1, c->Ep};
-    k_elem<<<dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), fS ? 2 : 1), ELEM_THREADS, 0,
-             c->stream>>>(jr, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1,
-                          c->bp2, (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
+    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), fS ? 2 : 1), ELEM_THREADS,
+              0, jr, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
+              (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     c->launches++;
     CO_CK(cudaGetLastError());
     return gather_solve_two(c, c->E, c->y, L, c->E, c->y, L, 1);
@@ -1084,9 +1095,9 @@ int co_compute_r_dev(co_ctx *c, const double *f, double *r) {
 
 int co_entropy_parts_dev(co_ctx *c, const double *f) {
     co_elem_job js = {f, 1, c->Ep};
-    k_elem<<<dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), 1), ELEM_THREADS, 0, c->stream>>>(
-        js, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
-        (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
+    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), 1), ELEM_THREADS, 0, js, js,
+              c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
+              (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     c->launches++;
     CO_CK(cudaGetLastError());
     return CO_OK;
@@ -1129,9 +1140,8 @@ int co_grad_L_dev(co_ctx *c, const double *x, int N, const double *L, double *G,
                   const double *w, double *dS, const double *dv, double *red) {
     if (N == 0) return CO_OK;
     co_lambda_job none = {};
-    k_grad_L<<<red_grid(c, N), CO_RED_THREADS, 0, c->stream>>>(
-        x, N, c->mb.cell, c->mb.xi, L, c->n1, c->nd1, c->ih1, c->ih2, c->P1, c->P2, G, w, dS, dv,
-        red, none);
+    co_launch(c, k_grad_L, red_grid(c, N), CO_RED_THREADS, 0, x, N, c->mb.cell, c->mb.xi, L, c->n1,
+              c->nd1, c->ih1, c->ih2, c->P1, c->P2, G, w, dS, dv, red, none);
     c->launches++;
     CO_CK(cudaGetLastError());
     return CO_OK;
@@ -1142,9 +1152,8 @@ int co_grad_L_lambda_dev(co_ctx *c, const double *x, int N, const double *L, dou
                          double S0, int gonzalez, const double *Ep) {
     if (N == 0) return CO_ERR_ARG;
     co_lambda_job lam = {c->st, S0, gonzalez, Ep, c->n_el, c->tickets + CO_TICKET_LAMBDA};
-    k_grad_L<<<red_grid(c, N), CO_RED_THREADS, 0, c->stream>>>(
-        x, N, c->mb.cell, c->mb.xi, L, c->n1, c->nd1, c->ih1, c->ih2, c->P1, c->P2, G, w, dS, dv,
-        red, lam);
+    co_launch(c, k_grad_L, red_grid(c, N), CO_RED_THREADS, 0, x, N, c->mb.cell, c->mb.xi, L, c->n1,
+              c->nd1, c->ih1, c->ih2, c->P1, c->P2, G, w, dS, dv, red, lam);
     c->launches++;
     CO_CK(cudaGetLastError());
     return CO_OK;
@@ -1153,8 +1162,8 @@ int co_grad_L_lambda_dev(co_ctx *c, const double *x, int N, const double *L, dou
 int co_loggrad_dev(co_ctx *c, const double *x, int N, const double *f, double *g,
                    const double *w, const double *dv, double *red) {
     if (N == 0) return CO_OK;
-    k_loggrad<<<red_grid(c, N), CO_RED_THREADS, 0, c->stream>>>(
-        x, N, c->mb.cell, c->mb.xi, f, c->n1, c->nd1, c->bp1, c->bp2, c->C1, c->C2, g, w, dv, red);
+    co_launch(c, k_loggrad, red_grid(c, N), CO_RED_THREADS, 0, x, N, c->mb.cell, c->mb.xi, f,
+              c->n1, c->nd1, c->bp1, c->bp2, c->C1, c->C2, g, w, dv, red);
     c->launches++;
     CO_CK(cudaGetLastError());
     return CO_OK;
