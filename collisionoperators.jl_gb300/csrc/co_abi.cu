@@ -456,6 +456,7 @@ static int check_opts(const co_opts *o) {
 static int collision_common(co_ctx *c, const double *v, const double *w, const double *G,
                             double *dot_v, int N) {
     ENTER(c);
+    co_fixed_scope fx(c);
     if (N < 0 || (N > 0 && (!v || !w || !G || !dot_v))) return CO_ERR_ARG;
     if (N == 0) return CO_OK;
     if (!all_finite(v, 2 * (size_t)N) || !all_finite(w, N) || !all_finite(G, 2 * (size_t)N))
@@ -482,6 +483,7 @@ extern "C" int co_collision(co_ctx *c, const double *v, const double *w, const d
 extern "C" int co_collision_metric(co_ctx *c, const double *v, const double *w, const double *G,
                                    double *dot_v, double *A, int N) {
     ENTER(c);
+    co_fixed_scope fx(c);
     if (N < 0 || (N > 0 && (!v || !w || !G || !dot_v || !A))) return CO_ERR_ARG;
     if (N == 0) return CO_OK;
     RC(co_ensure_capacity(c, N, 2));
@@ -570,6 +572,7 @@ extern "C" int co_mass_solve(co_ctx *c, const double *rhs, double *out) {
 extern "C" int co_picard_map(co_ctx *c, const co_opts *o, double *v_out, const double *v_in,
                              const double *v0, const double *w, int N, double S0, double dt) {
     ENTER(c);
+    co_fixed_scope fx(c);
     RC(check_opts(o));
     if (N < 0 || (N > 0 && (!v_out || !v_in || !v0 || !w))) return CO_ERR_ARG;
     if (N == 0) return CO_OK;

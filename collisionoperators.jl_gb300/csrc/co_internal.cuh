@@ -162,7 +162,8 @@ struct co_ctx {
     struct co_prof *prof;
     unsigned long long maps64, maps32, mapsds;
     // batch membership (co_batch): marker count and whether the instance has a pair sum
-    int batch_N, batch_landau, batch_member;
+    int batch_N, batch_landau;
+    int fixed_ok;              // FP64 pair sums may take the fixed-point form (co_fixed_scope)
     int lb_two_pass;          // LB drift in two launches (capturable) instead of cooperative
     // bounded grid barrier of the cooperative LB kernel: polls before it gives
     // up with CO_ERR_TIMEOUT, and phantom blocks it waits for on top of the
@@ -278,14 +279,21 @@ static inline int co_pack_mode(int precision) {
 }
 // Whether an FP64-accurate pair sum of up to Mub markers takes the fixed-point
 // kernel: from four 128-marker tiles on; below that the one-sided FP64 kernel's
-// single launch is as fast. The one-sided FP64 form also stays for CO_FLAG_ONESIDED,
-// and the batch engine keeps the FP64 form: a solve that stagnates returns an iterate
-// that round-off decides, and in a sample of batches 3 of 14 held such an instance,
-// whose result moved by 1e-6 to 1e-4 under the fixed-point sums.
+// single launch is as fast. The one-sided FP64 form also stays for CO_FLAG_ONESIDED.
+// Calls that evaluate the sum once take it (co_fixed_scope). A solve repeats it, and on a
+// stiff map the iteration multiplies a difference of 1e-16 until the solve stops at
+// another iterate (3 of 40 steps of 10,000 markers, 3 of 14 batches, by 1e-6 to 1e-4):
+// solves and the predictor, from which they start, keep the FP64 form, but for the
+// first iterations of step_anderson! (FIXED_ITERS).
 static inline int co_use_fixed(const co_ctx *c, int Mub, int precision) {
     return (precision == CO_PREC_FP64 || precision == CO_PREC_BOTH) && c->pair_symmetric &&
-           !c->batch_member && co_cdiv(Mub, 128) >= 4;
+           c->fixed_ok && co_cdiv(Mub, 128) >= 4;
 }
+struct co_fixed_scope {
+    co_ctx *c;
+    explicit co_fixed_scope(co_ctx *c_) : c(c_) { c->fixed_ok = 1; }
+    ~co_fixed_scope() { c->fixed_ok = 0; }
+};
 // operands of the fixed-point pair sum, as the kernels take them
 struct co_fixed_ops {
     const longlong2 *x;     // coordinates

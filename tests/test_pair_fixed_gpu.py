@@ -78,3 +78,26 @@ def test_scalings_are_exact(built_lib, collops_mod, oracle_mod, lo, hi):
     assert rel(ref, om.collision(v, w, G)) < TOL
     assert np.array_equal(run(w * 2.0 ** -300, G) * 2.0 ** 300, ref)
     assert np.array_equal(run(w, G * 2.0 ** 400) * 2.0 ** -400, ref)
+
+
+@pytest.mark.parametrize("max_iter,tol,done", [(200, 1e-9, True), (70, 0.0, False)])
+def test_solve_restarts(built_lib, collops_mod, oracle_mod, max_iter, tol, done):
+    """step_anderson! starts on the fixed-point sums and, where they do not converge
+    soon, again from the same guess in FP64: both ends against the oracle. The solve
+    stops at 1e-9 of |v|, or after 70 maps well below that; bound 1e-8."""
+    N = 700
+    v, w = gaussian_markers(N, 1.0, 0.6, seed=9)
+    bp = uniform_bp(-6.0, 6.0, 8)
+    om = oracle_mod.OracleMesh(bp, bp, 6)
+    o = oracle_mod.Opts(m=5, max_iter=max_iter, tol=tol, abs_floor=0.0, damping=0.7,
+                        stag_window=1000)
+    S0 = om.entropy(om.l2_project(v, w))
+    guess = om.predictor(o, v, w, 0.01)
+    ref = om.step_anderson(o, guess, v, w, S0, 0.01)
+    ws = collops_mod.build_workspace(collops_mod.SimParameters(bp1=bp, bp2=bp))
+    out = guess.copy(order="F")
+    it = collops_mod.step_anderson(ws, out, v, w, S0, 0.01, m=5, max_iter=max_iter, tol=tol,
+                                   abs_floor=0.0, damping=0.7, stag_window=1000)
+    ws.close()
+    assert (it[0] < max_iter) is done
+    assert rel(out, ref[0]) < 1e-8
