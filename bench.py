@@ -527,6 +527,9 @@ def run_gpu(args, cfg):
                "k_pair_ds_sym")
     r64 = roof(prof64.pair64_ms, prof64.pair64_launches, prof64.pair64_pairs, peak64.value,
                "fp64", "k_pair64_sym")
+    if r64:
+        r64["note"] = ("k_pair64_sym, and k_pair_fixed_sym (64-bit fixed point on the integer "
+                       "pipes) in the first iterations of the solve; the average is over both")
     if rds:
         rds["fp64_equivalent_frac"] = round(rds["achieved"] / (peak64.value / 1e12), 3)
         rds["note"] = ("double-single (FP32 head+tail) arithmetic: 23 FP64-equivalent flops per "
