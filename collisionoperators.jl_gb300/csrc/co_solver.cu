@@ -855,9 +855,9 @@ static int anderson_loop(co_ctx *c, const co_opts *o, int precision, int N, doub
 }
 
 // Iterations that step_anderson! gives the fixed-point pair sums before it starts again
-// in FP64. 57 of 60 steps of 10,000 markers converge within 48, in 10 to 46 iterations,
-// 1.7e-12 and less from the FP64 solve (11 iterations: 28.9 -> 5.8 ms); the other three
-// pay 24 ms of 240 to 395 for the attempt.
+// in FP64. 245 of 260 steps of 10,000 markers converge within 48, in 10 to 46 iterations,
+// 1.7e-12 and less from the FP64 solve (11 iterations: 28.9 -> 5.8 ms); the others, which
+// cannot be told by their residuals earlier, pay 20 to 24 ms for the attempt, on 130 to 430.
 #define FIXED_ITERS 48
 
 // step_anderson! on device buffers: mb.v1 (guess in, solution out), mb.v0, mb.w
