@@ -163,6 +163,9 @@ __device__ __forceinline__ void fixed_group(fixed_smem<W, NC> &sm, const co_fixe
                 if (SRC) sm.acc[i][j] = fma(v[i], o.pwn[ig], sm.acc[i][j]);
             }
         }
+        // the source's sum passes on: lane - 1 may add to it in the next step, and the
+        // shuffles below do not order shared memory between lanes
+        if (SRC) __syncwarp();
         // a close pair adds nothing here
         const int rs = 32 - d.s, src = (lane + 1) & 31;
 #pragma unroll
@@ -178,7 +181,6 @@ __device__ __forceinline__ void fixed_group(fixed_smem<W, NC> &sm, const co_fixe
         }
     }
     if (SRC) {
-        __syncwarp();   // close pairs of other lanes have added to this lane's sources
         const int k = grp * 32 + lane;
 #pragma unroll
         for (int i = 0; i < NC; i++) sm.acc[i][k] = fma(tf[i > 1], fx_to_double(b[i]), sm.acc[i][k]);
