@@ -67,11 +67,12 @@ struct co_bufs {
     float4 *pf_g;        // {g1h, g2h, g1l, g2l}
     float *pf_w, *pf_wl; // weight head / tail
     // fixed-point operands of the FP64-accurate pair sum (co_pair_fixed.cu): X1, X2
-    // per marker, G in limbs, the scaled weights (also as FP64),
-    // the scales {into, out of} the scaled units, and the pack kernel's block
-    // maxima (|G|, |w|)
+    // per marker, G in limbs, what their rounding left (X1 X2 G1 G2), the scaled
+    // weights (also as FP64), the scales {into, out of} the scaled units, and the pack
+    // kernel's block maxima (|G|, |w|)
     long long *fx_x, *fx_w;
-    int4 *fx_g;
+    int4 *fx_g, *fx_rest;
+    int4 *fx_box;        // bounds {min, max} of the high words of 32 markers each
     double *pwn, *unit;
     double2 *gwmax;
     double *pdot;        // packed vdot (2 x cap)
@@ -298,10 +299,14 @@ struct co_fixed_scope {
 struct co_fixed_ops {
     const longlong2 *x;     // coordinates
     const int4 *g;          // gradients: two limbs per component
+    const int4 *rest;       // what the rounding of x and g left
+    const int4 *box;        // bounds of the high words of 32 markers each
     const long long *w;     // weights
     const double2 *px, *pg; // FP64 operands (close pairs)
     const double *pwn, *unit;
     float m_close;          // a pair whose larger |d| component is below takes the FP64 form
+    float m_small;          // from three words
+    int x_near;             // bounds of x closer than this: a pair may be below m_small
 };
 int co_pair_fixed_pack(co_ctx *c, int Mub, int npart);  // px, pg, pw -> fixed-point operands
 int co_pair_fixed_sum(co_ctx *c, int Mub, int metric, int prof_kind);  // -> pdot (and pA)

@@ -4,6 +4,7 @@
 //   coordinate  X = x' 2^61, |x'| < 1           (two's complement, 64 bits)
 //   gradient    G = G' 2^60 = gh 2^31 + gl,     |G'| < 1, |gl| <= 2^30
 //   weight      w = w' 2^61, |w'| <= 1
+// and what the rounding of X and G left, in units of 2^-32 of theirs (32 bits)
 // A 64-bit product's high part comes from 32 x 32 -> 64 multiply-adds (one
 // IMAD.WIDE each) on limbs of base 2^31, whose cross terms fit a signed 64-bit
 // sum without a carry. Right shifts of cross terms round to nearest: the added
@@ -66,11 +67,12 @@ FXF uint32_t fx_seed(int32_t rhi) {
 #endif
 }
 
-// D = X_a - X_g shifted left until its larger component fills 61 bits
-struct fx_dist {
-    fx_limb d1, d2;   // normalised, base 2^31, half the shifted value
+// A difference (of coordinates or gradients) shifted left until its larger component
+// fills 61 bits
+struct fx_diff {
+    fx_limb c1, c2;   // normalised, base 2^31, half the shifted value
     int s;            // the shift
-    float m;          // size of the unshifted larger component (2^29 for |D'| = 1)
+    float m;          // size of the unshifted larger component (2^29 for 2^61)
 };
 FXF fx_limb fx_shl(fx64 d, int s) {
 #ifdef __CUDA_ARCH__
@@ -82,20 +84,47 @@ FXF fx_limb fx_shl(fx64 d, int s) {
     return {fx_hi(x), (int32_t)(fx_lo(x) >> 1)};
 #endif
 }
-FXF fx_dist fx_norm(fx64 D1, fx64 D2) {
-    fx_dist r;
-    const float f1 = fx_i2f(fx_hi(D1)), f2 = fx_i2f(fx_hi(D2));
-    r.m = fmaxf(fabsf(f1), fabsf(f2));
+FXF int fx_shift_of(float m) {   // 29 - exponent
 #ifdef __CUDA_ARCH__
-    r.s = (int)((0x4e7fffffu - __float_as_uint(r.m)) >> 23);   // 29 - exponent
+    const uint32_t b = __float_as_uint(m);
 #else
     uint32_t b;
-    memcpy(&b, &r.m, 4);
-    r.s = (int)((0x4e7fffffu - b) >> 23);
+    memcpy(&b, &m, 4);
 #endif
-    r.d1 = fx_shl(D1, r.s);
-    r.d2 = fx_shl(D2, r.s);
-    return r;
+    return (int)((0x4e7fffffu - b) >> 23);
+}
+FXF float fx_size(fx64 D1, fx64 D2) {
+    return fmaxf(fabsf(fx_i2f(fx_hi(D1))), fabsf(fx_i2f(fx_hi(D2))));
+}
+FXF fx_diff fx_norm(fx64 D1, fx64 D2) {
+    const float m = fx_size(D1, D2);
+    const int s = fx_shift_of(m);
+    return {fx_shl(D1, s), fx_shl(D2, s), s, m};
+}
+
+// 96-bit value h + l 2^-32
+struct fx96 {
+    fx64 h;
+    uint32_t l;
+};
+// difference of the rounded words and of what their rounding left
+FXF fx96 fx_sub96(fx64 D, int32_t ra, int32_t rg) {
+    const fx64 r = (fx64)ra - rg;
+    return {D + (r >> 32), fx_lo(r)};
+}
+FXF fx_limb fx_shl(fx96 d, int s) {   // 0 <= s < 32
+#ifdef __CUDA_ARCH__
+    const uint32_t l = __funnelshift_l(d.l, fx_lo(d.h), s);
+    return {(int32_t)__funnelshift_l(fx_lo(d.h), (uint32_t)fx_hi(d.h), s), (int32_t)(l >> 1)};
+#else
+    const fxu64 x = ((fxu64)d.h << s) | (((fxu64)d.l << s) >> 32);
+    return {fx_hi((fx64)x), (int32_t)(fx_lo((fx64)x) >> 1)};
+#endif
+}
+FXF fx_diff fx_norm(fx96 D1, fx96 D2) {
+    const float m = fx_size(D1.h, D2.h);
+    const int s = fx_shift_of(m);
+    return {fx_shl(D1, s), fx_shl(D2, s), s, m};
 }
 
 // y3 = |d|^-3 of the normalised distance: y^3 2^58 (y = r^-1/2, r = d1^2 + d2^2
@@ -112,7 +141,7 @@ FXF fx_limb fx_invcube(const fx_limb &d1, const fx_limb &d2) {
     const fxu64 W = fx_mulu(V, Y, 0x8c0000000ull);      // r Y^2: (1 + e) 2^56 + 8.75
     const int32_t e = fx_mid((fx64)W, 4);               // e 2^52, |e| < 2^-21.6
     // y^3 (1 + e)^-3/2 = y^3 (1 + c), c = e (-3/2 + 15/8 e) + O(e^3 ~ 2^-64)
-    const int32_t P = fx_hi(fx_mad(e, 1920, -(3ll << 61)));       // (-3/2 + 15/8 e) 2^30
+    const int32_t P = fx_hi(fx_mad(e, 1920, (1ll << 31) - (3ll << 61)));       // (-3/2 + 15/8 e) 2^30
     const int32_t c = fx_mid(fx_mad(e, P, 1ll << 29), 30);         // c 2^52
     const fxu64 Q = fx_madu(Y, Y, 0);
     const fx64 Y3 = (fx64)fx_mulu(Q, Y, 0);             // Y^3 2^-32
@@ -121,13 +150,40 @@ FXF fx_limb fx_invcube(const fx_limb &d1, const fx_limb &d2) {
 }
 
 // C = K1 D2 + nK2 D1 (nK2 = G_g2 - G_a2), times 2^-62
-FXF fx64 fx_cross(int32_t k1h, int32_t k1l, int32_t k2h, int32_t k2l, const fx_limb &d1,
-                  const fx_limb &d2) {
-    fx64 x = fx_mad(k1h, d2.l, 1ll << 30);
-    x = fx_mad(k1l, d2.h, x);
-    x = fx_mad(k2h, d1.l, x);
-    x = fx_mad(k2l, d1.h, x);
-    fx64 C = fx_mad(k1h, d2.h, 0);
-    C = fx_mad(k2h, d1.h, C);
+FXF fx64 fx_cross(const fx_limb &k1, const fx_limb &k2, const fx_limb &d1, const fx_limb &d2) {
+    fx64 x = fx_mad(k1.h, d2.l, 1ll << 30);
+    x = fx_mad(k1.l, d2.h, x);
+    x = fx_mad(k2.h, d1.l, x);
+    x = fx_mad(k2.l, d1.h, x);
+    fx64 C = fx_mad(k1.h, d2.h, 0);
+    C = fx_mad(k2.h, d1.h, C);
     return fx_mad(fx_hi(x), 2, C);
+}
+// -2^n <= a, b < 2^n
+FXF bool fx_within(int32_t a, int32_t b, int n) {
+    return (((uint32_t)(a + (1 << n)) | (uint32_t)(b + (1 << n))) >> (n + 1)) == 0;
+}
+FXF fx64 fx_join(const fx_limb &a) { return ((fx64)a.h << 31) + a.l; }
+
+// A pair's differences from all 96 bits, K normalised like D, so that the error of its
+// terms is relative to its own |d| and |g|. K's shift stays below D's, sf = d.s + 1 - it:
+// terms are then no finer than the unit their sums have, 2^-57 of the scales.
+struct fx_fine {
+    fx_diff d;
+    fx_limb k1, k2;
+    int sf;   // shift of the terms of S
+};
+FXF fx_fine fx_refine(fx96 D1, fx96 D2, fx96 K1, fx96 K2) {
+    fx_fine p;
+    p.d = fx_norm(D1, D2);
+    const int k = fx_shift_of(fx_size(K1.h, K2.h)), s = k < p.d.s + 1 ? k : p.d.s + 1;
+    p.k1 = fx_shl(K1, s);
+    p.k2 = fx_shl(K2, s);
+    p.sf = p.d.s + 1 - s;
+    return p;
+}
+// the same from the rounded words alone
+FXF fx_fine fx_plain(fx64 D1, fx64 D2, const fx_limb &k1, const fx_limb &k2) {
+    const fx_diff d = fx_norm(D1, D2);
+    return {d, k1, k2, d.s};
 }

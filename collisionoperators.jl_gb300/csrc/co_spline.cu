@@ -1217,9 +1217,11 @@ int co_ensure_capacity(co_ctx *c, int N, int m) {
         if ((rc = grow(&b.pf_w, (size_t)cap))) return rc;
         if ((rc = grow(&b.pf_wl, (size_t)cap))) return rc;
         // fixed-point operands: one allocation (cap is a multiple of 256)
-        if ((rc = grow(&b.fx_x, 6 * (size_t)cap + (size_t)cap / 128 + 4))) return rc;
+        if ((rc = grow(&b.fx_x, 8 * (size_t)cap + (size_t)cap / 8 + (size_t)cap / 128 + 4))) return rc;
         b.fx_g = (int4 *)(b.fx_x + n2);
-        b.fx_w = (long long *)(b.fx_g + cap);
+        b.fx_rest = b.fx_g + cap;
+        b.fx_box = b.fx_rest + cap;
+        b.fx_w = (long long *)(b.fx_box + cap / 16);
         b.pwn = (double *)(b.fx_w + cap);
         b.gwmax = (double2 *)(b.pwn + cap);
         b.unit = (double *)(b.gwmax + cap / 256);

@@ -1,0 +1,114 @@
+"""FP64 pair sums and metric over wide ranges of the operands, marker by marker, against
+sums in extended precision: coordinates far below the size of the domain, close pairs
+near the origin, clusters of small G.
+
+Bound: at most twice the error of the one-sided FP64 kernels on the same inputs. An error
+is taken relative to the sizes of a marker's terms, w_a |G_a - G_g| / |d| (the metric:
+w_a / |d|), and of all markers the largest counts; below two units of 2^-53 (the rounding
+of the final sum) any error will do.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import gaussian_markers
+
+pytestmark = pytest.mark.gpu
+
+
+def sums(v, w, G):
+    """F, A and the sizes of their terms, in extended precision (N x 2, N x 3, N, N)."""
+    L = np.longdouble
+    v, w, G = v.astype(L), w.astype(L), G.astype(L)
+    N = len(w)
+    F, A, sf, sa = np.zeros((N, 2), L), np.zeros((N, 3), L), np.zeros(N, L), np.zeros(N, L)
+    for i in range(0, N, 100):
+        s = slice(i, i + 100)
+        d1, d2 = v[s, None, 0] - v[:, 0], v[s, None, 1] - v[:, 1]
+        g1, g2 = G[:, 0] - G[s, None, 0], G[:, 1] - G[s, None, 1]
+        r2 = d1 * d1 + d2 * d2
+        r = np.where(r2 < 1e-24, np.inf, np.sqrt(r2))
+        k = w / (r * r * r)
+        c = k * (g1 * d2 - g2 * d1)
+        F[s] = np.stack([(c * d2).sum(1), -(c * d1).sum(1)], 1)
+        A[s] = np.stack([(k * d2 * d2).sum(1), -(k * d1 * d2).sum(1), (k * d1 * d1).sum(1)], 1)
+        sf[s] = (np.abs(w) * np.sqrt(g1 * g1 + g2 * g2) / r).sum(1)
+        sa[s] = (np.abs(w) / r).sum(1)
+    return F, A, sf, sa
+
+
+def check(collops, bp, v, w, G):
+    N = len(w)
+    v, G = np.asfortranarray(v), np.asfortranarray(G)
+    Fr, Ar, sf, sa = sums(v, w, G)
+    err = {}
+    for onesided in (True, False):
+        ws = collops.build_workspace(
+            collops.SimParameters(bp1=bp, bp2=bp, pair_onesided=onesided))
+        dv, F, A = (np.zeros((N, k), order="F") for k in (2, 2, 3))
+        collops.compute_collision_gpu(ws, dv, v, w, G)
+        collops.compute_collision_metric_gpu(ws, F, A, v, w, G)
+        ws.close()
+        err[onesided] = [float(np.max(np.abs(got - ref) / size[:, None])) for got, ref, size in
+                         ((dv, Fr, sf), (F, Fr, sf), (A, Ar, sa))]
+    for here, fp64 in zip(err[False], err[True]):
+        assert here <= max(2 * fp64, 2.0 ** -52)
+
+
+def graded(half):
+    return np.concatenate([np.linspace(-6.0, 6.0, 13)] if half == 6.0 else
+                          [[-half], np.linspace(-6.0, 6.0, 13), [half]])
+
+
+def _markers(N, seed, weights="random"):
+    v, w = gaussian_markers(N, 1.0, 0.6, seed=seed)
+    rng = np.random.default_rng(seed)
+    if weights == "random":
+        w = rng.uniform(0.2, 1.8, N) / N
+    G = -v / [1.0, 0.36] + 0.2 * np.sin(2 * v[:, ::-1]) + 0.05 * rng.standard_normal(v.shape)
+    return v, w, G
+
+
+@pytest.mark.parametrize("weights", ["equal", "random"])
+@pytest.mark.parametrize("half", [6.0, 1e2, 1e4, 1e6])
+def test_wide_domains(built_lib, collops_mod, half, weights):
+    """Markers of thermal width 1 in domains of larger and larger half-width."""
+    check(collops_mod, graded(half), *_markers(1200, 3, weights))
+
+
+@pytest.mark.parametrize("gap", [4.1e-6, 4e-5, 1e-3])
+def test_close_pairs_near_the_origin(built_lib, collops_mod, gap):
+    """Pairs beyond the reach of the FP64 form whose coordinates are all small."""
+    v, w, G = _markers(1200, 5)
+    rng = np.random.default_rng(8)
+    v[:200] = 0.05 * (rng.random((200, 2)) - 0.5)
+    t = rng.uniform(0, 2 * np.pi, 100)
+    v[100:200] = v[:100] + gap * np.stack([np.cos(t), np.sin(t)], 1)
+    check(collops_mod, graded(6.0), v, w, G)
+
+
+@pytest.mark.parametrize("share", [2, 10])
+@pytest.mark.parametrize("k", [6, 12, 18])
+def test_cold_core(built_lib, collops_mod, k, share):
+    """A share of the markers 2^k times colder than the rest, with a smooth G."""
+    v, w, G = _markers(1200, 7)
+    v[::share] *= 2.0 ** -k
+    G[::share] *= 2.0 ** -k
+    check(collops_mod, graded(6.0), v, w, G)
+
+
+def test_tiny_domain(built_lib, collops_mod, oracle_mod):
+    """A domain so small that the guard distance 1e-12 is far beyond the usual reach of the
+    FP64 form. Against the CPU oracle: sums of N FP64 terms, ten times sqrt(N) 2^-53."""
+    v, w, G = _markers(1200, 9)
+    v = np.asfortranarray(v * 2.0 ** -38)
+    G = np.asfortranarray(G)
+    bp = graded(6.0) * 2.0 ** -38
+    ws = collops_mod.build_workspace(collops_mod.SimParameters(bp1=bp, bp2=bp))
+    F, A = np.zeros((1200, 2), order="F"), np.zeros((1200, 3), order="F")
+    collops_mod.compute_collision_metric_gpu(ws, F, A, v, w, G)
+    ws.close()
+    Fr, Ar = oracle_mod.OracleMesh(bp, bp, 6).collision_metric(v, w, G)
+    for got, ref in ((F, Fr), (A, Ar)):
+        assert np.max(np.abs(got - ref)) <= 10 * 1200 ** 0.5 * 2.0 ** -53 * np.max(np.abs(ref))
