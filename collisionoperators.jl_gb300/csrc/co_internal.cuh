@@ -39,6 +39,7 @@ struct co_solver_state {
     int path;            // 0 damped Picard, 1 Anderson, for the current k
     int improved;        // nrm_r < nrm_best at the current k
     int error;           // device-detected error (non-finite residual, timeout)
+    int wide;            // the last operands' range was too wide for fixed-point sums
     double nrm_r0, nrm_r, nrm_v, nrm_best, nrm_best_window, damp, res_out;
     double best32;       // defect correction: best FP32-stage outer residual
     int kbest32;         // and the outer map that reached it
@@ -302,8 +303,9 @@ struct co_fixed_ops {
     const int4 *rest;       // what the rounding of x and g left
     const int4 *box;        // bounds of the high words of 32 markers each
     const long long *w;     // weights
-    const double2 *px, *pg; // FP64 operands (close pairs)
-    const double *pwn, *unit;
+    const double2 *px, *pg; // FP64 operands
+    const double *pw, *pwn, *unit;
+    const int *wide;        // take all pairs in FP64
     float m_close;          // a pair whose larger |d| component is below takes the FP64 form
     float m_small;          // from three words
     int x_near;             // bounds of x closer than this: a pair may be below m_small

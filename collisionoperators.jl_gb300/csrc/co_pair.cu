@@ -29,21 +29,10 @@
 // partial sums are accumulated in FP64.
 #include "co_f32x2.cuh"
 #include "co_internal.cuh"
+#include "co_pair64.cuh"
 #include "co_reduce.cuh"
 
 #define PAIR_TPB 128
-
-// bit pattern of 1e-24 (functions.jl:224 guard)
-#define CO_R2_MIN_BITS 0x3B282DB34012B251LL
-
-__device__ __forceinline__ double rsqrt_seed64(double x) {
-    // FP32 value of x from its high word (x in [1e-30, 1e30], positive)
-    int hi = __double2hiint(x);
-    float xf = __int_as_float((hi - (896 << 20)) << 3);
-    float yf = rsqrtf(xf);
-    int fb = __float_as_int(yf);
-    return __hiloint2double((fb >> 3) + (896 << 20), fb << 29);
-}
 
 __device__ __forceinline__ void pair64(double xg1, double xg2, double Gg1, double Gg2,
                                        double xa1, double xa2, double Ga1, double Ga2,
@@ -320,33 +309,6 @@ k_metric32(const float4 *__restrict__ pfx, const float *__restrict__ pfw,
 // 23 per unordered pair, 11.5 per ordered pair (20 in k_pair64).
 #define ST 128
 
-__device__ __forceinline__ void pair_u64(double d1, double d2, double g1, double g2, double &u1,
-                                         double &u2) {
-    double r2 = d1 * d1;
-    r2 = fma(d2, d2, r2);
-    bool ok = __double_as_longlong(r2) >= CO_R2_MIN_BITS;
-    double xr = ok ? r2 : 1.0;
-    double y = rsqrt_seed64(xr);
-    double t = xr * y;
-    double e = fma(-t, y, 1.0);
-    double p = fma(0.375, e, 0.5);
-    double ye = y * e;
-    y = fma(ye, p, y);
-    double dg = d1 * g1;
-    dg = fma(d2, g2, dg);
-    double y2 = y * y;
-    double cc = dg * y2;
-    double t1 = fma(-d1, cc, g1);
-    double t2 = fma(-d2, cc, g2);
-    double ym = ok ? y : 0.0;
-    u1 = t1 * ym;
-    u2 = t2 * ym;
-}
-
-__device__ __forceinline__ bool sym_skip(int nt, int H, int I, int k) {
-    return k > 0 && (nt & 1) == 0 && k == H && I >= nt / 2;
-}
-
 // The FP64 pair sum of solves and predictors; batch instances run the same arithmetic in
 // k_pair64_sym_batch. Bound by the FP64 pipe (89 % of its peak; 10,000 markers 2.1 ms
 // against 0.36 of the fixed-point form).
@@ -354,63 +316,10 @@ __global__ void __launch_bounds__(ST)
 k_pair64_sym(const double2 *__restrict__ px, const double2 *__restrict__ pg,
              const double *__restrict__ pw, int nt, int H, int KC,
              double *__restrict__ gpart, double *__restrict__ apart) {
-    __shared__ double2 sx[ST], sg[ST];
-    __shared__ double sw[ST];
-    __shared__ double2 sacc[ST];
-    const int I = blockIdx.x % nt, chunk = blockIdx.x / nt;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const double2 xg = px[I * ST + tid], Gg = pg[I * ST + tid];
-    const double wg = pw[I * ST + tid];
-    double ga1 = 0.0, ga2 = 0.0;
-    const int k0 = chunk * KC, k1 = min(H + 1, k0 + KC);
-    for (int k = k0; k < k1; k++) {
-        if (sym_skip(nt, H, I, k)) continue;
-        const int J = (I + k) % nt;
-        __syncthreads();
-        sx[tid] = px[J * ST + tid];
-        sg[tid] = pg[J * ST + tid];
-        sw[tid] = pw[J * ST + tid];
-        sacc[tid] = make_double2(0.0, 0.0);
-        __syncthreads();
-        if (k == 0) {  // diagonal tile: ordered pairs, self excluded by the guard
-#pragma unroll 4
-            for (int a = 0; a < ST; a++) {
-                double u1, u2;
-                double2 xa = sx[a], Ga = sg[a];
-                pair_u64(xg.x - xa.x, xg.y - xa.y, Ga.x - Gg.x, Ga.y - Gg.y, u1, u2);
-                ga1 = fma(sw[a], u1, ga1);
-                ga2 = fma(sw[a], u2, ga2);
-            }
-            continue;
-        }
-        for (int r = 0; r < 4; r++) {
-            const int base = ((warp + r) & 3) * 32;
-            double2 a0 = sacc[base + lane];
-            double a1 = a0.x, a2 = a0.y;
-#pragma unroll 4
-            for (int q = 0; q < 32; q++) {
-                const int ai = base + ((lane + q) & 31);
-                double2 xa = sx[ai], Ga = sg[ai];
-                double wa = sw[ai];
-                double u1, u2;
-                pair_u64(xg.x - xa.x, xg.y - xa.y, Ga.x - Gg.x, Ga.y - Gg.y, u1, u2);
-                ga1 = fma(wa, u1, ga1);
-                ga2 = fma(wa, u2, ga2);
-                a1 = fma(-wg, u1, a1);
-                a2 = fma(-wg, u2, a2);
-                a1 = __shfl_sync(0xffffffffu, a1, (lane + 1) & 31);
-                a2 = __shfl_sync(0xffffffffu, a2, (lane + 1) & 31);
-            }
-            sacc[base + lane] = make_double2(a1, a2);
-            __syncthreads();
-        }
-        double *ap = apart + ((size_t)(k - 1) * nt + J) * 2 * ST;
-        ap[tid] = sacc[tid].x;
-        ap[ST + tid] = sacc[tid].y;
-    }
-    double *gp = gpart + ((size_t)chunk * nt + I) * 2 * ST;
-    gp[tid] = ga1;
-    gp[ST + tid] = ga2;
+    __shared__ sym64_smem<4, 2> sm;
+    const int I = blockIdx.x % nt, chunk = blockIdx.x / nt, k0 = chunk * KC;
+    sym64_item<4, 2>(sm, px, pg, pw, nt, H, I, k0, min(H + 1, k0 + KC),
+                     gpart + ((size_t)chunk * nt + I) * 2 * ST, apart);
 }
 
 // FP32 body on head/tail operands: returns the unweighted term u
@@ -1143,6 +1052,7 @@ struct co_pack_out {
     float4 *pfx, *pfg;
     float *pfw, *pfwl;
     double2 *gwmax;   // block maxima of |G| and |w| (the fixed-point scales)
+    int *wide;        // co_solver_state::wide, cleared for the fixed-point operands
 };
 
 __device__ __forceinline__ void pack_store(const co_pack_out &o, int mode, int p, bool in,
@@ -1182,6 +1092,7 @@ __device__ __forceinline__ void pack_max(const co_pack_out &o, double x1, double
             wm = fmax(wm, sh[i].y);
         }
         o.gwmax[blockIdx.x] = make_double2(gm, wm);
+        if (blockIdx.x == 0) *o.wide = 0;
     }
 }
 
@@ -1428,7 +1339,7 @@ int co_pair_fp32(co_ctx *c, int Mub) {
 
 static co_pack_out pack_out(co_ctx *c) {
     co_bufs &b = c->mb;
-    return {b.px, b.pg, b.pw, b.pf_x, b.pf_g, b.pf_w, b.pf_wl, b.gwmax};
+    return {b.px, b.pg, b.pw, b.pf_x, b.pf_g, b.pf_w, b.pf_wl, b.gwmax, &c->st->wide};
 }
 
 int co_pack_plain(co_ctx *c, int N, int Mub, int precision, const double *x, const double *G) {
@@ -1537,14 +1448,10 @@ template <int W>
 __global__ void __launch_bounds__(32 * W)
 k_pair64_sym_batch(const co_bwork *__restrict__ works, int n_inst, int total, int KC,
                    unsigned *__restrict__ counter) {
-    constexpr int T = 32 * W;
-    __shared__ double2 sx[T], sg[T];
-    __shared__ double sw[T];
-    __shared__ double2 sacc[T];
+    __shared__ sym64_smem<W, 2> sm;
     __shared__ int s_item;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(counter, 1u);
+        if (threadIdx.x == 0) s_item = (int)atomicAdd(counter, 1u);
         __syncthreads();
         const int item = s_item;
         __syncthreads();
@@ -1556,61 +1463,10 @@ k_pair64_sym_batch(const co_bwork *__restrict__ works, int n_inst, int total, in
         }
         const co_bwork wk = works[lo];
         if (wk.st->done) continue;
-        const int b = item - wk.blk0;
-        const int nt = wk.nt, H = wk.H;
-        const int I = b % nt, chunk = b / nt;
-        const double2 xg = wk.px[I * T + tid], Gg = wk.pg[I * T + tid];
-        const double wg = wk.pw[I * T + tid];
-        double ga1 = 0.0, ga2 = 0.0;
-        const int k0 = chunk * KC, k1 = min(H + 1, k0 + KC);
-        for (int k = k0; k < k1; k++) {
-            if (sym_skip(nt, H, I, k)) continue;
-            const int J = (I + k) % nt;
-            __syncthreads();
-            sx[tid] = wk.px[J * T + tid];
-            sg[tid] = wk.pg[J * T + tid];
-            sw[tid] = wk.pw[J * T + tid];
-            sacc[tid] = make_double2(0.0, 0.0);
-            __syncthreads();
-            if (k == 0) {
-#pragma unroll 4
-                for (int a = 0; a < T; a++) {
-                    double u1, u2;
-                    double2 xa = sx[a], Ga = sg[a];
-                    pair_u64(xg.x - xa.x, xg.y - xa.y, Ga.x - Gg.x, Ga.y - Gg.y, u1, u2);
-                    ga1 = fma(sw[a], u1, ga1);
-                    ga2 = fma(sw[a], u2, ga2);
-                }
-                continue;
-            }
-            for (int r = 0; r < W; r++) {
-                const int base = ((warp + r) % W) * 32;
-                double2 a0 = sacc[base + lane];
-                double a1 = a0.x, a2 = a0.y;
-#pragma unroll 4
-                for (int q = 0; q < 32; q++) {
-                    const int ai = base + ((lane + q) & 31);
-                    double2 xa = sx[ai], Ga = sg[ai];
-                    double wa = sw[ai];
-                    double u1, u2;
-                    pair_u64(xg.x - xa.x, xg.y - xa.y, Ga.x - Gg.x, Ga.y - Gg.y, u1, u2);
-                    ga1 = fma(wa, u1, ga1);
-                    ga2 = fma(wa, u2, ga2);
-                    a1 = fma(-wg, u1, a1);
-                    a2 = fma(-wg, u2, a2);
-                    a1 = __shfl_sync(0xffffffffu, a1, (lane + 1) & 31);
-                    a2 = __shfl_sync(0xffffffffu, a2, (lane + 1) & 31);
-                }
-                sacc[base + lane] = make_double2(a1, a2);
-                __syncthreads();
-            }
-            double *ap = wk.apart + ((size_t)(k - 1) * nt + J) * 2 * T;
-            ap[tid] = sacc[tid].x;
-            ap[T + tid] = sacc[tid].y;
-        }
-        double *gp = wk.gpart + ((size_t)chunk * nt + I) * 2 * T;
-        gp[tid] = ga1;
-        gp[T + tid] = ga2;
+        const int b = item - wk.blk0, nt = wk.nt, H = wk.H;
+        const int I = b % nt, chunk = b / nt, k0 = chunk * KC;
+        sym64_item<W, 2>(sm, wk.px, wk.pg, wk.pw, nt, H, I, k0, min(H + 1, k0 + KC),
+                         wk.gpart + ((size_t)chunk * nt + I) * 64 * W, wk.apart);
     }
 }
 

@@ -44,13 +44,19 @@
 // The metric A = sum_a w_a U(v_g - v_a) of functions.jl:249-290 comes from the same
 // evaluation: U = (d2, -d1) (d2, -d1)^T / |d|^3.
 //
+// Range: where the operands of a launch span too much for one scale (fixed_wide), the
+// same tiles run the FP64 pair term (co_pair64.cuh) instead, on the device's own decision:
+// 16,384 markers 5.8 ms, with the metric 9.2.
+//
 // Tiling: tiles of TS = 32 W sorted markers, W warps, one target per lane; tile
 // pairs (I, I + k mod nt), k = 0..nt/2, so each unordered tile pair appears once
 // and one evaluation serves both markers (Newton's third law). Within a warp,
 // lane l meets source (l + q) mod 32 of a 32-source group at step q, and the
 // source's accumulators pass to lane l - 1 by shuffles. Partials go to fixed slots
 // and are added in a fixed order: bitwise reproducible.
+#include "co_f32x2.cuh"
 #include "co_internal.cuh"
+#include "co_pair64.cuh"
 #include "co_pair_fixed.cuh"
 
 // 96-bit sum of terms T 2^s
@@ -219,10 +225,6 @@ __device__ __forceinline__ void fixed_group(fixed_smem<W, NC> &sm, const co_fixe
     }
 }
 
-__device__ __forceinline__ bool fixed_skip(int nt, int H, int I, int k) {
-    return k > 0 && (nt & 1) == 0 && k == H && I >= nt / 2;
-}
-
 // sign of sum i in the target's and the source's result
 __device__ __forceinline__ double fixed_sign(int i, bool src) {
     return i == 0 ? (src ? -1.0 : 1.0) : i == 1 ? (src ? 1.0 : -1.0) : i == 3 ? -1.0 : 1.0;
@@ -230,13 +232,13 @@ __device__ __forceinline__ double fixed_sign(int i, bool src) {
 
 // tile I against tiles I + k, k0 <= k < k1
 template <int W, int NC>
-__device__ __forceinline__ void fixed_item(fixed_smem<W, NC> &sm, const co_fixed_ops &o, int nt,
-                                           int H, int I, int k0, int k1, double *__restrict__ gp,
+__device__ __forceinline__ void fixed_item(fixed_smem<W, NC> &sm, const co_fixed_ops &o,
+                                           const fixed_target &t, int nt, int H, int I, int k0,
+                                           int k1, double *__restrict__ gp,
                                            double *__restrict__ apart) {
     constexpr int TS = 32 * W;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ig = I * TS + tid;
-    const fixed_target t = {o.x[ig], o.g[ig], o.w[ig]};
     // the equal-weight loop serves tile pairs whose markers all carry weight w0
     const fx64 w0 = o.w[(size_t)I * TS];
     const bool own = w0 != 0 && t.w == w0;
@@ -245,7 +247,7 @@ __device__ __forceinline__ void fixed_item(fixed_smem<W, NC> &sm, const co_fixed
     for (int i = 0; i < NC; i++) gd[i] = 0.0;
 #pragma unroll 1
     for (int k = k0; k < k1; k++) {
-        if (fixed_skip(nt, H, I, k)) continue;
+        if (sym_skip(nt, H, I, k)) continue;
         int J = I + k;
         if (J >= nt) J -= nt;
         __syncthreads();
@@ -292,15 +294,21 @@ __device__ __forceinline__ void fixed_item(fixed_smem<W, NC> &sm, const co_fixed
 }
 
 template <int W, int NC>
-__global__ void __launch_bounds__(32 * W)
+__global__ void __launch_bounds__(32 * W, NC == 2 ? (W == 4 ? 7 : 25) : 16 / W)
 k_pair_fixed_sym(const co_fixed_ops o, int nt, int H, int KC, double *__restrict__ gpart,
                  double *__restrict__ apart) {
     co_grid_wait();
-    __shared__ fixed_smem<W, NC> sm;
+    __shared__ union {
+        fixed_smem<W, NC> f;
+        sym64_smem<W, NC> d;
+    } sm;
     const int I = blockIdx.x % nt, chunk = blockIdx.x / nt;
     const int k0 = chunk * KC, k1 = min(H + 1, k0 + KC);
-    fixed_item<W, NC>(sm, o, nt, H, I, k0, k1, gpart + ((size_t)chunk * nt + I) * 32 * W * NC,
-                      apart);
+    double *gp = gpart + ((size_t)chunk * nt + I) * 32 * W * NC;
+    const int ig = I * 32 * W + threadIdx.x;
+    const fixed_target t = {o.x[ig], o.g[ig], o.w[ig]};
+    if (*o.wide) sym64_item<W, NC>(sm.d, o.px, o.pg, o.pw, nt, H, I, k0, k1, gp, apart);
+    else fixed_item<W, NC>(sm.f, o, t, nt, H, I, k0, k1, gp, apart);
 }
 
 // The sums of the packed positions: the target-side partials of every chunk and
@@ -313,13 +321,15 @@ k_pair_fixed_sym(const co_fixed_ops o, int nt, int H, int KC, double *__restrict
 template <int NC>
 __global__ void __launch_bounds__(32 * FIXED_SL)
 k_fixed_reduce(const double *__restrict__ gpart, const double *__restrict__ apart, int nt, int H,
-               int nchunk, int TS, const double *__restrict__ unit, double *__restrict__ pdot,
-               double *__restrict__ pA, size_t ld) {
+               int nchunk, int TS, const double *__restrict__ unit, const int *__restrict__ wide,
+               double *__restrict__ pdot, double *__restrict__ pA, size_t ld) {
     co_grid_wait();
     __shared__ double sh[NC][FIXED_SL][33];
     const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const int p = blockIdx.x * 32 + lane;          // TS is a multiple of 32
     const int K = p / TS, t = p - K * TS;
+    // FP64 sums have no scale
+    const double u = sl >= NC || *wide ? 1.0 : unit[sl < 2 ? 1 : 3];
     double s[NC];
 #pragma unroll
     for (int i = 0; i < NC; i++) s[i] = 0.0;
@@ -332,7 +342,7 @@ k_fixed_reduce(const double *__restrict__ gpart, const double *__restrict__ apar
     for (int k = 1 + sl; k <= H; k += FIXED_SL) {
         int I = K - k;
         if (I < 0) I += nt;
-        if (fixed_skip(nt, H, I, k)) continue;
+        if (sym_skip(nt, H, I, k)) continue;
         const double *ap = apart + ((size_t)(k - 1) * nt + K) * NC * TS + t;
 #pragma unroll
         for (int i = 0; i < NC; i++) s[i] += ap[i * TS];
@@ -344,8 +354,8 @@ k_fixed_reduce(const double *__restrict__ gpart, const double *__restrict__ apar
         double r = sh[sl][0][lane];
 #pragma unroll
         for (int i = 1; i < FIXED_SL; i++) r += sh[sl][i][lane];
-        if (sl < 2) pdot[(size_t)sl * ld + p] = r * unit[1];
-        else pA[(size_t)(sl - 2) * ld + p] = r * unit[3];
+        if (sl < 2) pdot[(size_t)sl * ld + p] = r * u;
+        else pA[(size_t)(sl - 2) * ld + p] = r * u;
     }
 }
 
@@ -356,6 +366,41 @@ __device__ __forceinline__ int scale_exp(double x) {
     if (!(x > 0.0)) return 0;
     const int e = ilogb(x) + 1;
     return e < -1000 ? -1000 : (e > 1000 ? 1000 : e);
+}
+
+// Whether the fixed-point sums of a marker would be less accurate than FP64 ones. Their
+// terms w |g| / |d| are accurate relative to |g| / |d|, but rounded to 2^-57 of the largest
+// G and to 2^-61 of the largest weight, so one marker of a huge G, or of a weight far
+// above the others', costs the sums of all others digits. Against that stands the sum
+// itself, estimated from 64 of the sorted markers (scaled: largest G and weight about 1;
+// 1/|d| counts up to 64, so that one close sample does not decide). The fixed-point form
+// stays while w |g| / |d| is on average above 2^-6 of what the units stand for: its error
+// is then below that of FP64 arithmetic for every marker (a weightless marker of |G| 2^k
+// times the others: 2^-2 to 2^-5.5 and 0.1 to 0.7 times FP64's error for k = 0 to 5, 2^-6.4
+// and 1.2 times for k = 6). Thermal distributions with the solver's own G: 2^-4 and more.
+// Markers so close together in their domain that most pairs would be close ones are left
+// to the FP64 loop too (half-width 1e6 for thermal width 1). 2 us of a map of 2,048 markers.
+#define FIXED_SAMPLES 64
+__device__ __forceinline__ bool fixed_wide(const float4 *sv, const float *swt, float x1, float x2,
+                                           float G1, float G2, bool force) {
+    float num = 0.f, gr = 0.f, wr = 0.f, rr = 0.f;
+    int near = 0;
+#pragma unroll 4
+    for (int s = 0; s < FIXED_SAMPLES; s++) {
+        const float4 v = sv[s];
+        const float d1 = x1 - v.x, d2 = x2 - v.y, g1 = G1 - v.z, g2 = G2 - v.w;
+        const float r2 = fmaf(d2, d2, d1 * d1);
+        near += r2 < 0x1p-40f;
+        const float r = r2 > 0.f ? fminf(rsqrt_normal(r2), 64.f) : 0.f;   // 0: the marker itself
+        const float gg = fmaf(g2, g2, fmaf(g1, g1, 0x1p-80f));
+        const float q = gg * rsqrt_normal(gg) * r;
+        num = fmaf(swt[s], q, num);
+        gr += q;
+        wr = fmaf(swt[s], r, wr);
+        rr += r;
+    }
+    const bool ok = (!force || num >= 0x1p-6f * (gr + FIXED_SAMPLES)) && wr >= 0x1p-6f * rr;
+    return !ok || near > FIXED_SAMPLES / 8;
 }
 
 // a rounded to an integer, and what that leaves in units of 2^-32
@@ -372,13 +417,15 @@ __device__ __forceinline__ fx64 fx_round(double a, int &rest) {
 // scaled units; unit[1], unit[3]: scaled sums back to vdot and A.
 __global__ void __launch_bounds__(256)
 k_pair_fixed_pack(const double2 *__restrict__ px, const double2 *__restrict__ pg,
-                  const double *__restrict__ pw, const int *__restrict__ Mp, int Mpad,
+                  const double *__restrict__ pw, const int *__restrict__ Mp,
                   const double2 *__restrict__ part, int npart, int ex, double c1, double c2,
                   longlong2 *__restrict__ ox, int4 *__restrict__ og, int4 *__restrict__ rest,
                   int4 *__restrict__ box, fx64 *__restrict__ ow, double *__restrict__ pwn,
-                  double *__restrict__ unit) {
+                  double *__restrict__ unit, int *__restrict__ wide) {
     co_grid_wait();
     __shared__ double shg[8], shw[8];
+    __shared__ float4 sv[FIXED_SAMPLES];   // x1 x2 g1 g2, scaled
+    __shared__ float swt[FIXED_SAMPLES];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double gm = 0.0, wm = 0.0;
     for (int i = tid; i < npart; i += blockDim.x) {
@@ -408,11 +455,18 @@ k_pair_fixed_pack(const double2 *__restrict__ px, const double2 *__restrict__ pg
         unit[2] = ldexp(1.0, ex);
         unit[3] = ok ? ldexp(1.0, ew - ex) : nan("");
     }
-    const int p = blockIdx.x * blockDim.x + tid;
-    if (p >= Mpad) return;
+    const int M = *Mp;
+    if (tid < FIXED_SAMPLES && M > 0) {
+        const int q = (int)((long long)tid * M / FIXED_SAMPLES);
+        const double2 x = px[q], G = pg[q];
+        sv[tid] = make_float4((float)((x.x - c1) * sx), (float)((x.y - c2) * sx), (float)(G.x * sg),
+                              (float)(G.y * sg));
+        swt[tid] = (float)fabs(pw[q] * sw);
+    }
+    const int p = blockIdx.x * blockDim.x + tid;   // below Mpad: the blocks are whole
     // padding: outside the scaled domain (coordinates stay below 1/2), weight 0
     double x1 = 0.96875, x2 = 0.96875, G1 = 0.0, G2 = 0.0, wn = 0.0;
-    if (p < *Mp) {
+    if (p < M) {
         const double2 x = px[p], G = pg[p];
         x1 = (x.x - c1) * sx;
         x2 = (x.y - c2) * sx;
@@ -434,10 +488,12 @@ k_pair_fixed_pack(const double2 *__restrict__ px, const double2 *__restrict__ pg
     lo.z = __reduce_min_sync(0xffffffffu, hw[2]), hi.z = __reduce_max_sync(0xffffffffu, hw[2]);
     lo.w = __reduce_min_sync(0xffffffffu, hw[3]), hi.w = __reduce_max_sync(0xffffffffu, hw[3]);
     if (lane < 2) box[2 * (p >> 5) + lane] = lane ? hi : lo;
+    __syncthreads();
+    const bool bad = p < M && fixed_wide(sv, swt, (float)x1, (float)x2, (float)G1, (float)G2, gm > 0.0);
+    if (__syncthreads_or(bad) && tid == 0) *wide = 1;   // every writer writes the same
     og[p] = make_int4(h1, (int)(V1 - ((fx64)h1 << 31)), h2, (int)(V2 - ((fx64)h2 << 31)));
-    const fx64 w = __double2ll_rn(wn * 0x1p61);
-    ow[p] = w;
-    pwn[p] = (double)w * 0x1p-61;
+    ow[p] = __double2ll_rn(wn * 0x1p61);
+    pwn[p] = wn;
 }
 
 // ------------------------------------------------------------------ host
@@ -459,9 +515,9 @@ int co_pair_fixed_pack(co_ctx *c, int Mub, int npart) {
     const int ex = ilogb(big) + 2;
     c->fixed_ex = ex;
     const int Mpad = co_cdiv(Mub, 256) * 256;
-    co_launch(c, k_pair_fixed_pack, Mpad / 256, 256, 0, b.px, b.pg, b.pw, b.cstart + c->n_el, Mpad,
+    co_launch(c, k_pair_fixed_pack, Mpad / 256, 256, 0, b.px, b.pg, b.pw, b.cstart + c->n_el,
               b.gwmax, npart, ex, c1, c2, (longlong2 *)b.fx_x, b.fx_g, b.fx_rest,
-              b.fx_box, b.fx_w, b.pwn, b.unit);
+              b.fx_box, b.fx_w, b.pwn, b.unit, &c->st->wide);
     c->launches++;
     CO_CK(cudaGetLastError());
     return CO_OK;
@@ -477,7 +533,9 @@ co_fixed_ops co_fixed_operands(co_ctx *c) {
     o.w = b.fx_w;
     o.px = b.px;
     o.pg = b.pg;
+    o.pw = b.pw;
     o.pwn = b.pwn;
+    o.wide = &c->st->wide;
     o.unit = b.unit;
     // |d| < 2^-22 in scaled units, and at least the 1e-12 guard distance, in units
     // of the coordinates' high words (2^29 for 1)
@@ -516,7 +574,7 @@ static int fixed_run(co_ctx *c, int Mub, int KC, int prof_kind) {
               gpart, apart);
     co_prof_end(c);
     co_launch(c, k_fixed_reduce<NC>, nt * W, 32 * FIXED_SL, 0, gpart, apart, nt, H, nchunk, TS,
-              c->mb.unit, c->mb.pdot, c->mb.pA, (size_t)c->mb.cap);
+              c->mb.unit, &c->st->wide, c->mb.pdot, c->mb.pA, (size_t)c->mb.cap);
     c->launches += 2;
     CO_CK(cudaGetLastError());
     return CO_OK;

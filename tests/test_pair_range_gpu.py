@@ -112,3 +112,65 @@ def test_tiny_domain(built_lib, collops_mod, oracle_mod):
     Fr, Ar = oracle_mod.OracleMesh(bp, bp, 6).collision_metric(v, w, G)
     for got, ref in ((F, Fr), (A, Ar)):
         assert np.max(np.abs(got - ref)) <= 10 * 1200 ** 0.5 * 2.0 ** -53 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("size", [1e2, 1e3, 1e5, 1e8, 1e12, 1e17])
+@pytest.mark.parametrize("weight", [0.0, 1e-14])
+def test_one_huge_gradient(built_lib, collops_mod, weight, size):
+    """A marker of (next to) no weight with a G far above the others': it adds nothing to
+    them and must not cost them digits."""
+    v, w, G = _markers(1200, 11)
+    w[400] *= weight
+    G[400, 0] = size
+    check(collops_mod, graded(6.0), v, w, G)
+
+
+@pytest.mark.parametrize("ratio", [1e1, 1e2, 1e4, 1e12])
+def test_one_heavy_marker(built_lib, collops_mod, ratio):
+    v, w, G = _markers(1200, 13)
+    w /= ratio
+    w[700] = 1.0 / 1200
+    check(collops_mod, graded(6.0), v, w, G)
+
+
+@pytest.mark.parametrize("balanced", [False, True])
+@pytest.mark.parametrize("decades", [2, 4, 12])
+def test_weights_over_decades(built_lib, collops_mod, decades, balanced):
+    """Weights log-uniform over decades, with G of one size or balanced, G ~ 1/w."""
+    v, w, G = _markers(1200, 17)
+    s = 10.0 ** (-decades * np.random.default_rng(4).random(1200))
+    w *= s
+    if balanced:
+        G /= s[:, None]
+    check(collops_mod, graded(6.0), v, w, G)
+
+
+@pytest.mark.parametrize("offset", [1e2, 1e4, 1e8])
+def test_common_part_of_the_gradient(built_lib, collops_mod, offset):
+    """Only differences of G count."""
+    v, w, G = _markers(1200, 19)
+    check(collops_mod, graded(6.0), v, w, G + [offset, -0.3 * offset])
+
+
+def test_map_of_unequal_weights(built_lib, collops_mod, oracle_mod):
+    """The map forms lambda dv / w itself, so weights over twelve decades give a G over as
+    many: a marker's error against the CPU oracle at most twice that of the one-sided FP64
+    kernels, or one unit of 2^-52 of its velocity."""
+    N = 1200
+    v, w, _ = _markers(N, 23)
+    w = w * 10.0 ** (-12 * np.random.default_rng(6).random(N))
+    v = np.asfortranarray(v)
+    v_in = np.asfortranarray(v - 0.01 * v + 0.001 * np.sin(3 * v[:, ::-1]))
+    bp = np.linspace(-6.0, 6.0, 13)
+    om = oracle_mod.OracleMesh(bp, bp, 6)
+    S0 = om.entropy(om.l2_project(v, w))
+    ref = om.picard_map(oracle_mod.Opts(), v_in, v, w, S0, 0.01)
+    err = {}
+    for onesided in (True, False):
+        ws = collops_mod.build_workspace(
+            collops_mod.SimParameters(bp1=bp, bp2=bp, pair_onesided=onesided))
+        out = np.zeros((N, 2), order="F")
+        collops_mod.picard_map(ws, out, v_in, v, w, S0, 0.01)
+        ws.close()
+        err[onesided] = float(np.max(np.linalg.norm(out - ref, axis=1) / np.linalg.norm(ref, axis=1)))
+    assert err[False] <= max(2 * err[True], 2.0 ** -52)
