@@ -318,7 +318,7 @@ k_pair64_sym(const double2 *__restrict__ px, const double2 *__restrict__ pg,
              double *__restrict__ gpart, double *__restrict__ apart) {
     __shared__ sym64_smem<4, 2> sm;
     const int I = blockIdx.x % nt, chunk = blockIdx.x / nt, k0 = chunk * KC;
-    sym64_item<4, 2>(sm, px, pg, pw, nt, H, I, k0, min(H + 1, k0 + KC),
+    sym64_item<4, 2>(sm, px, pg, pw, nt, H, I, k0, min(H + 1, k0 + KC), 1,
                      gpart + ((size_t)chunk * nt + I) * 2 * ST, apart);
 }
 
@@ -1465,7 +1465,7 @@ k_pair64_sym_batch(const co_bwork *__restrict__ works, int n_inst, int total, in
         if (wk.st->done) continue;
         const int b = item - wk.blk0, nt = wk.nt, H = wk.H;
         const int I = b % nt, chunk = b / nt, k0 = chunk * KC;
-        sym64_item<W, 2>(sm, wk.px, wk.pg, wk.pw, nt, H, I, k0, min(H + 1, k0 + KC),
+        sym64_item<W, 2>(sm, wk.px, wk.pg, wk.pw, nt, H, I, k0, min(H + 1, k0 + KC), 1,
                          wk.gpart + ((size_t)chunk * nt + I) * 64 * W, wk.apart);
     }
 }

@@ -58,12 +58,12 @@ struct sym64_smem {
 };
 
 // Tile I of T = 32 W markers against the tiles I + k, k0 <= k < k1, one target per
-// thread: target sums to gp, the sources' to their slots in apart
+// thread: target sums to gp, the sources' to their slots in apart (the first is ka's)
 template <int W, int NC>
 __device__ __forceinline__ void sym64_item(sym64_smem<W, NC> &sm, const double2 *__restrict__ px,
                                            const double2 *__restrict__ pg,
                                            const double *__restrict__ pw, int nt, int H, int I,
-                                           int k0, int k1, double *__restrict__ gp,
+                                           int k0, int k1, int ka, double *__restrict__ gp,
                                            double *__restrict__ apart) {
     constexpr int T = 32 * W;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -117,7 +117,7 @@ __device__ __forceinline__ void sym64_item(sym64_smem<W, NC> &sm, const double2 
             for (int i = 0; i < NC; i++) sm.acc[i][base + lane] = b[i];
             __syncthreads();
         }
-        double *ap = apart + ((size_t)(k - 1) * nt + J) * NC * T;
+        double *ap = apart + ((size_t)(k - ka) * nt + J) * NC * T;
 #pragma unroll
         for (int i = 0; i < NC; i++) ap[i * T + tid] = sm.acc[i][tid];
     }

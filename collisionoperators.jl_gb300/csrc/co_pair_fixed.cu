@@ -234,7 +234,7 @@ __device__ __forceinline__ double fixed_sign(int i, bool src) {
 template <int W, int NC>
 __device__ __forceinline__ void fixed_item(fixed_smem<W, NC> &sm, const co_fixed_ops &o,
                                            const fixed_target &t, int nt, int H, int I, int k0,
-                                           int k1, double *__restrict__ gp,
+                                           int k1, int ka, double *__restrict__ gp,
                                            double *__restrict__ apart) {
     constexpr int TS = 32 * W;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -282,7 +282,7 @@ __device__ __forceinline__ void fixed_item(fixed_smem<W, NC> &sm, const co_fixed
             }
         }
         if (k > 0) {
-            double *ap = apart + ((size_t)(k - 1) * nt + J) * NC * TS;
+            double *ap = apart + ((size_t)(k - ka) * nt + J) * NC * TS;
 #pragma unroll
             for (int i = 0; i < NC; i++) ap[i * TS + tid] = fixed_sign(i, true) * sm.acc[i][tid];
         }
@@ -295,25 +295,26 @@ __device__ __forceinline__ void fixed_item(fixed_smem<W, NC> &sm, const co_fixed
 
 template <int W, int NC>
 __global__ void __launch_bounds__(32 * W, NC == 2 ? (W == 4 ? 7 : 25) : 16 / W)
-k_pair_fixed_sym(const co_fixed_ops o, int nt, int H, int KC, double *__restrict__ gpart,
-                 double *__restrict__ apart) {
+k_pair_fixed_sym(const co_fixed_ops o, int nt, int H, int KC, int kb, int ke,
+                 double *__restrict__ gpart, double *__restrict__ apart) {
     co_grid_wait();
     __shared__ union {
         fixed_smem<W, NC> f;
         sym64_smem<W, NC> d;
     } sm;
     const int I = blockIdx.x % nt, chunk = blockIdx.x / nt;
-    const int k0 = chunk * KC, k1 = min(H + 1, k0 + KC);
+    const int k0 = kb + chunk * KC, k1 = min(ke, k0 + KC), ka = max(kb, 1);
     double *gp = gpart + ((size_t)chunk * nt + I) * 32 * W * NC;
     const int ig = I * 32 * W + threadIdx.x;
     const fixed_target t = {o.x[ig], o.g[ig], o.w[ig]};
-    if (*o.wide) sym64_item<W, NC>(sm.d, o.px, o.pg, o.pw, nt, H, I, k0, k1, gp, apart);
-    else fixed_item<W, NC>(sm.f, o, t, nt, H, I, k0, k1, gp, apart);
+    if (*o.wide) sym64_item<W, NC>(sm.d, o.px, o.pg, o.pw, nt, H, I, k0, k1, ka, gp, apart);
+    else fixed_item<W, NC>(sm.f, o, t, nt, H, I, k0, k1, ka, gp, apart);
 }
 
 // The sums of the packed positions: the target-side partials of every chunk and
-// the source-side partials of every k, in a fixed order, times the unit of the
-// scaled operands; components 0, 1 to vdot and 2.. to A. FIXED_SL threads share a
+// the source-side partials of ka <= k < ke, in a fixed order, times the unit of the
+// scaled operands; components 0, 1 to vdot and 2.. to A, added to what is there where
+// add is set. FIXED_SL threads share a
 // position (a slice of the rows each), so a small launch does not wait on one
 // chain of loads, and the FP64 rounding of the sum grows with the slice's length
 // instead of the row count.
@@ -321,8 +322,9 @@ k_pair_fixed_sym(const co_fixed_ops o, int nt, int H, int KC, double *__restrict
 template <int NC>
 __global__ void __launch_bounds__(32 * FIXED_SL)
 k_fixed_reduce(const double *__restrict__ gpart, const double *__restrict__ apart, int nt, int H,
-               int nchunk, int TS, const double *__restrict__ unit, const int *__restrict__ wide,
-               double *__restrict__ pdot, double *__restrict__ pA, size_t ld) {
+               int nchunk, int ka, int ke, int TS, const double *__restrict__ unit,
+               const int *__restrict__ wide, int add, double *__restrict__ pdot,
+               double *__restrict__ pA, size_t ld) {
     co_grid_wait();
     __shared__ double sh[NC][FIXED_SL][33];
     const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
@@ -339,11 +341,11 @@ k_fixed_reduce(const double *__restrict__ gpart, const double *__restrict__ apar
         for (int i = 0; i < NC; i++) s[i] += gp[i * TS];
     }
 #pragma unroll 4
-    for (int k = 1 + sl; k <= H; k += FIXED_SL) {
+    for (int k = ka + sl; k < ke; k += FIXED_SL) {
         int I = K - k;
         if (I < 0) I += nt;
         if (sym_skip(nt, H, I, k)) continue;
-        const double *ap = apart + ((size_t)(k - 1) * nt + K) * NC * TS + t;
+        const double *ap = apart + ((size_t)(k - ka) * nt + K) * NC * TS + t;
 #pragma unroll
         for (int i = 0; i < NC; i++) s[i] += ap[i * TS];
     }
@@ -354,8 +356,8 @@ k_fixed_reduce(const double *__restrict__ gpart, const double *__restrict__ apar
         double r = sh[sl][0][lane];
 #pragma unroll
         for (int i = 1; i < FIXED_SL; i++) r += sh[sl][i][lane];
-        if (sl < 2) pdot[(size_t)sl * ld + p] = r * u;
-        else pA[(size_t)(sl - 2) * ld + p] = r * u;
+        double *d = sl < 2 ? pdot + (size_t)sl * ld + p : pA + (size_t)(sl - 2) * ld + p;
+        *d = add ? fma(r, u, *d) : r * u;
     }
 }
 
@@ -562,20 +564,31 @@ static void fixed_shape(co_ctx *c, int Mub, int *W, int *KC) {
     *KC = kc;
 }
 
+// Source-side partials take a slot per marker and k, N^2 / 256 in all (F with the metric
+// of 131,072 markers: 2.7 GB, of 2^20: 172). From FIXED_PART bytes on, the sum goes in
+// bands of k that fit, one after another on the same buffer.
+#define FIXED_PART (1ull << 30)
 template <int W, int NC>
 static int fixed_run(co_ctx *c, int Mub, int KC, int prof_kind) {
-    const int TS = 32 * W, nt = co_cdiv(Mub, TS), H = nt / 2, nchunk = co_cdiv(H + 1, KC);
-    const size_t gsz = (size_t)nchunk * nt * NC * TS;
-    int rc = co_ensure_part(c, gsz + (size_t)(H > 0 ? H : 1) * nt * NC * TS);
+    const int TS = 32 * W, nt = co_cdiv(Mub, TS), H = nt / 2;
+    const size_t row = (size_t)nt * NC * TS;   // slots of one k
+    const size_t fit = FIXED_PART / (8 * row) / KC * KC;
+    const int band = (size_t)H <= fit ? H + 1 : (int)(fit > 0 ? fit : KC);
+    const size_t gsz = co_cdiv(band, KC) * row;
+    int rc = co_ensure_part(c, gsz + (size_t)(band > H ? (H > 0 ? H : 1) : band) * row);
     if (rc) return rc;
     double *gpart = c->mb.part, *apart = c->mb.part + gsz;
     co_prof_begin(c, prof_kind);
-    co_launch(c, k_pair_fixed_sym<W, NC>, nt * nchunk, TS, 0, co_fixed_operands(c), nt, H, KC,
-              gpart, apart);
-    co_prof_end(c);
-    co_launch(c, k_fixed_reduce<NC>, nt * W, 32 * FIXED_SL, 0, gpart, apart, nt, H, nchunk, TS,
-              c->mb.unit, &c->st->wide, c->mb.pdot, c->mb.pA, (size_t)c->mb.cap);
-    c->launches += 2;
+    for (int kb = 0; kb <= H; kb += band) {
+        const int ke = kb + band < H + 1 ? kb + band : H + 1, nchunk = co_cdiv(ke - kb, KC);
+        co_launch(c, k_pair_fixed_sym<W, NC>, nt * nchunk, TS, 0, co_fixed_operands(c), nt, H, KC,
+                  kb, ke, gpart, apart);
+        if (ke == H + 1) co_prof_end(c);
+        co_launch(c, k_fixed_reduce<NC>, nt * W, 32 * FIXED_SL, 0, gpart, apart, nt, H, nchunk,
+                  kb > 0 ? kb : 1, ke, TS, c->mb.unit, &c->st->wide, (int)(kb > 0), c->mb.pdot,
+                  c->mb.pA, (size_t)c->mb.cap);
+        c->launches += 2;
+    }
     CO_CK(cudaGetLastError());
     return CO_OK;
 }
