@@ -144,7 +144,7 @@ static int spd_inverse(std::vector<double> A, int n, std::vector<double> &inv) {
 
 template <typename T>
 static int upload(T **dst, const std::vector<T> &src) {
-    if (cudaMalloc((void **)dst, src.size() * sizeof(T)) != cudaSuccess) return CO_ERR_NOMEM;
+    if (cudaMalloc((void **)dst, src.size() * sizeof(T)) != cudaSuccess) return co_nomem();
     if (cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess)
         return CO_ERR_CUDA;
     return CO_OK;
@@ -305,24 +305,24 @@ extern "C" int co_ctx_create(const double *bp1, int nb1, const double *bp2, int 
     TRY(upload(&c->Minv2, I2));
     double **cv[] = {&c->b, &c->y, &c->f, &c->fin, &c->rr, &c->L};
     for (double **p : cv)
-        if (cudaMalloc(p, sizeof(double) * c->n_dofs) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
-    if (cudaMalloc(&c->bS, sizeof(double) * 9 * c->n_el) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
-    if (cudaMalloc(&c->E, sizeof(double) * 9 * c->n_el) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
-    if (cudaMalloc(&c->Ep, sizeof(double) * c->n_el) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
-    if (cudaMalloc(&c->mb.count, sizeof(int) * c->n_el) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
-    if (cudaMalloc(&c->mb.cstart, sizeof(int) * (c->n_el + 1)) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
+        if (cudaMalloc(p, sizeof(double) * c->n_dofs) != cudaSuccess) { free_ctx(c); return co_nomem(); };
+    if (cudaMalloc(&c->bS, sizeof(double) * 9 * c->n_el) != cudaSuccess) { free_ctx(c); return co_nomem(); };
+    if (cudaMalloc(&c->E, sizeof(double) * 9 * c->n_el) != cudaSuccess) { free_ctx(c); return co_nomem(); };
+    if (cudaMalloc(&c->Ep, sizeof(double) * c->n_el) != cudaSuccess) { free_ctx(c); return co_nomem(); };
+    if (cudaMalloc(&c->mb.count, sizeof(int) * c->n_el) != cudaSuccess) { free_ctx(c); return co_nomem(); };
+    if (cudaMalloc(&c->mb.cstart, sizeof(int) * (c->n_el + 1)) != cudaSuccess) { free_ctx(c); return co_nomem(); };
     c->mb.red_cap = CO_RED_CAP;
     if (cudaMalloc(&c->mb.red, sizeof(double) * CO_RED_CAP * CO_RED_COMPS + 64) != cudaSuccess)
-        { free_ctx(c); return CO_ERR_NOMEM; };
-    if (cudaMalloc(&c->st, sizeof(co_solver_state)) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
+        { free_ctx(c); return co_nomem(); };
+    if (cudaMalloc(&c->st, sizeof(co_solver_state)) != cudaSuccess) { free_ctx(c); return co_nomem(); };
     if (cudaMalloc(&c->tickets, sizeof(unsigned) * CO_TICKETS) != cudaSuccess ||
         cudaMemset(c->tickets, 0, sizeof(unsigned) * CO_TICKETS) != cudaSuccess) {
         free_ctx(c);
-        return CO_ERR_NOMEM;
+        return co_nomem();
     }
-    if (cudaMallocHost(&c->st_host, sizeof(co_solver_state)) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
+    if (cudaMallocHost(&c->st_host, sizeof(co_solver_state)) != cudaSuccess) { free_ctx(c); return co_nomem(); };
     memset(c->st_host, 0, sizeof(co_solver_state));
-    if (cudaMallocHost(&c->bad_host, sizeof(int)) != cudaSuccess) { free_ctx(c); return CO_ERR_NOMEM; };
+    if (cudaMallocHost(&c->bad_host, sizeof(int)) != cudaSuccess) { free_ctx(c); return co_nomem(); };
     if (cudaMemset(c->st, 0, sizeof(co_solver_state)) != cudaSuccess) { free_ctx(c); return CO_ERR_CUDA; };
     TRY(co_spline_configure(c));
     TRY(co_ensure_capacity(c, 1024, 1));

@@ -209,6 +209,11 @@ static void co_launch(co_ctx *c, void (*k)(P...), dim3 grid, dim3 block, size_t 
 }
 
 // ------------------------------------------------------------- helpers
+// after a failed allocation: its error does not stay behind for the next call
+static inline int co_nomem() {
+    (void)cudaGetLastError();
+    return CO_ERR_NOMEM;
+}
 #define CO_CK(call)                                                   \
     do {                                                              \
         cudaError_t e_ = (call);                                      \

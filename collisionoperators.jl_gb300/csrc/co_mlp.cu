@@ -441,7 +441,7 @@ static int mlp_ensure(co_mlp *m, int nb) {
     m->cap = 0;
     if (cudaMalloc(&m->part, sizeof(float) * (size_t)nb * m->P) != cudaSuccess ||
         cudaMalloc(&m->lpart, sizeof(double) * nb + sizeof(float)) != cudaSuccess)
-        return CO_ERR_NOMEM;
+        return co_nomem();
     m->cap = nb;
     return CO_OK;
 }
@@ -476,7 +476,7 @@ extern "C" int co_mlp_create(int n_in, int n_out, unsigned seed, int device, co_
         cudaMalloc(&m->m1, sizeof(float) * o.P) != cudaSuccess ||
         cudaMalloc(&m->m2, sizeof(float) * o.P) != cudaSuccess) {
         co_mlp_destroy(m);
-        return CO_ERR_NOMEM;
+        return co_nomem();
     }
     cudaMemcpy(m->master, h.data(), sizeof(float) * o.P, cudaMemcpyHostToDevice);
     cudaMemset(m->m1, 0, sizeof(float) * o.P);
@@ -554,7 +554,7 @@ extern "C" int co_mlp_set_normalization(co_mlp *m, const double *x_mean, const d
         h[2 * MLP_MAX_IN + k] = (float)y_std[k];
         h[2 * MLP_MAX_IN + MLP_MAX_OUT + k] = (float)y_mean[k];
     }
-    if (!m->norm && cudaMalloc(&m->norm, sizeof(h)) != cudaSuccess) return CO_ERR_NOMEM;
+    if (!m->norm && cudaMalloc(&m->norm, sizeof(h)) != cudaSuccess) return co_nomem();
     CO_CK(cudaMemcpy(m->norm, h, sizeof(h), cudaMemcpyHostToDevice));
     return CO_OK;
 }

@@ -47,7 +47,7 @@ void co_newton_free(co_ctx *c) {
 static int nk_ensure(co_ctx *c, int N, int mem) {
     if (!c->nk) {
         c->nk = (co_nk_bufs *)calloc(1, sizeof(co_nk_bufs));
-        if (!c->nk) return CO_ERR_NOMEM;
+        if (!c->nk) return co_nomem();
     }
     co_nk_bufs *s = c->nk;
     if (N <= s->cap && mem <= s->mem && s->V) return CO_OK;
@@ -55,17 +55,17 @@ static int nk_ensure(co_ctx *c, int N, int mem) {
     int m = mem > s->mem ? mem : s->mem;
     co_newton_free(c);
     c->nk = (co_nk_bufs *)calloc(1, sizeof(co_nk_bufs));
-    if (!c->nk) return CO_ERR_NOMEM;
+    if (!c->nk) return co_nomem();
     s = c->nk;
     const size_t n2 = 2 * (size_t)cap * sizeof(double);
     double **v[] = {&s->F, &s->Ft, &s->xt, &s->xp, &s->Fp, &s->d, &s->xb, &s->Fb, &s->wv};
     for (double **p : v)
-        if (cudaMalloc(p, n2) != cudaSuccess) return CO_ERR_NOMEM;
+        if (cudaMalloc(p, n2) != cudaSuccess) return co_nomem();
     if (cudaMalloc(&s->V, n2 * (size_t)(m + 1)) != cudaSuccess ||
         cudaMalloc(&s->red, sizeof(double) * NK_RED) != cudaSuccess ||
         cudaMalloc(&s->scal, sizeof(double) * (m + 2)) != cudaSuccess ||
         cudaMalloc(&s->z, sizeof(double) * (m + 1)) != cudaSuccess)
-        return CO_ERR_NOMEM;
+        return co_nomem();
     s->cap = cap;
     s->mem = m;
     return CO_OK;

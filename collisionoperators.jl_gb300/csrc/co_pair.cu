@@ -1215,7 +1215,8 @@ int co_ensure_part(co_ctx *c, size_t n) {
     if (n <= c->mb.part_cap) return CO_OK;
     if (c->mb.part) cudaFree(c->mb.part);
     c->mb.part = nullptr;
-    if (cudaMalloc(&c->mb.part, n * sizeof(double)) != cudaSuccess) return CO_ERR_NOMEM;
+    c->mb.part_cap = 0;
+    if (cudaMalloc(&c->mb.part, n * sizeof(double)) != cudaSuccess) return co_nomem();
     c->mb.part_cap = n;
     return CO_OK;
 }

@@ -1257,31 +1257,31 @@ int co_step_defect_buffers(co_ctx *c, const co_opts *o, const co_defect_opts *do
         if (r0) *r0 = 0;
         return CO_OK;
     }
-    if (!c->st2 && cudaMalloc(&c->st2, sizeof(co_solver_state)) != cudaSuccess) return CO_ERR_NOMEM;
+    if (!c->st2 && cudaMalloc(&c->st2, sizeof(co_solver_state)) != cudaSuccess) return co_nomem();
     co_bufs &b = c->mb;
-    if (!b.Gk && cudaMalloc(&b.Gk, 2 * sizeof(double) * b.cap) != cudaSuccess) return CO_ERR_NOMEM;
-    if (!b.Phi && cudaMalloc(&b.Phi, 2 * sizeof(double) * b.cap) != cudaSuccess) return CO_ERR_NOMEM;
-    if (!b.Adef && cudaMalloc(&b.Adef, 3 * sizeof(double) * b.cap) != cudaSuccess) return CO_ERR_NOMEM;
+    if (!b.Gk && cudaMalloc(&b.Gk, 2 * sizeof(double) * b.cap) != cudaSuccess) return co_nomem();
+    if (!b.Phi && cudaMalloc(&b.Phi, 2 * sizeof(double) * b.cap) != cudaSuccess) return co_nomem();
+    if (!b.Adef && cudaMalloc(&b.Adef, 3 * sizeof(double) * b.cap) != cudaSuccess) return co_nomem();
     const int mo = dopt->outer_m;
     if (mo < 0 || mo > CO_MAX_M) return CO_ERR_ARG;
     const size_t ld2 = 2 * (size_t)b.cap;
     if (mo > 0) {
         if (!c->st3 && cudaMalloc(&c->st3, sizeof(co_solver_state)) != cudaSuccess)
-            return CO_ERR_NOMEM;
+            return co_nomem();
         if (b.aa && b.aa_m < mo) {
             cudaFree(b.aa);
             b.aa = nullptr;
         }
         if (!b.aa) {
             if (cudaMalloc(&b.aa, sizeof(double) * ld2 * (5 + 2 * (size_t)mo)) != cudaSuccess)
-                return CO_ERR_NOMEM;
+                return co_nomem();
             b.aa_m = mo;
         }
     }
     const int pcon = dopt->precond;
     if (pcon < 0 || pcon > 2) return CO_ERR_ARG;
     if (pcon && !b.pc && cudaMalloc(&b.pc, 7 * sizeof(double) * b.cap) != cudaSuccess)
-        return CO_ERR_NOMEM;
+        return co_nomem();
     double *pc_Psi = b.pc, *pc_z = b.pc ? b.pc + ld2 : nullptr,
            *pc_H = b.pc ? b.pc + 2 * ld2 : nullptr;
     double *aa_vk = b.aa, *aa_u = b.aa + ld2, *aa_r = b.aa + 2 * ld2, *aa_rp = b.aa + 3 * ld2,
@@ -1669,7 +1669,7 @@ extern "C" int co_batch_create(const co_batch_instance *inst, int n, int n_quad,
         cudaMalloc(&B->d_counter, 64) != cudaSuccess ||
         cudaMalloc(&B->d_loop, sizeof(int) * (n + 1)) != cudaSuccess) {
         co_batch_destroy(B);
-        return CO_ERR_NOMEM;
+        return co_nomem();
     }
     cudaMemset(B->st_all, 0, sizeof(co_solver_state) * n);
     size_t off = 0;
@@ -2116,9 +2116,9 @@ extern "C" int co_warmstart_features_dev(co_ctx *c, const co_opts *o, const doub
     if (res_pred) *res_pred = 0.0;
     if (N == 0) return CO_OK;
     co_bufs &b = c->mb;
-    if (!b.pc && cudaMalloc(&b.pc, 7 * sizeof(double) * b.cap) != cudaSuccess) return CO_ERR_NOMEM;
+    if (!b.pc && cudaMalloc(&b.pc, 7 * sizeof(double) * b.cap) != cudaSuccess) return co_nomem();
     if (!b.Adef && cudaMalloc(&b.Adef, 3 * sizeof(double) * b.cap) != cudaSuccess)
-        return CO_ERR_NOMEM;
+        return co_nomem();
     double *H = b.pc + 4 * (size_t)b.cap;   // 3N: the Hessian of L at v
     CO_CK(cudaMemcpyAsync(b.v0, v, 2 * (size_t)N * sizeof(double), cudaMemcpyDeviceToDevice,
                           c->stream));

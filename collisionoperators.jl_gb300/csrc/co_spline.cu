@@ -959,7 +959,7 @@ static int ensure_gs(co_ctx *c) {
               cudaMalloc(&g.y, sizeof(double) * c->n_dofs) == cudaSuccess;
     if (!ok) {
         co_sortset_free(c);
-        return CO_ERR_NOMEM;
+        return co_nomem();
     }
     c->gs_cap = c->mb.cap;
     return CO_OK;
@@ -1187,17 +1187,21 @@ static int grow(T **p, size_t n) {
     if (*p) cudaFree(*p);
     *p = nullptr;
     if (n == 0) n = 1;
-    if (cudaMalloc((void **)p, n * sizeof(T)) != cudaSuccess) return CO_ERR_NOMEM;
+    if (cudaMalloc((void **)p, n * sizeof(T)) != cudaSuccess) return co_nomem();
     return CO_OK;
 }
 
+// Where an allocation fails, the capacities stay 0 and the next call allocates anew: no
+// call finds a capacity whose buffers are not there.
 int co_ensure_capacity(co_ctx *c, int N, int m) {
     co_bufs &b = c->mb;
     int rc;
-    if (N > b.cap) {
+    if (N > b.cap || b.cap == 0) {
         int cap = N < 1024 ? 1024 : N;
         cap = (cap + 255) / 256 * 256;  // packed pair operands are padded to whole tiles
         size_t n2 = 2 * (size_t)cap;
+        const int m_cap = b.m_cap;
+        b.cap = b.m_cap = 0;
         double **d2[] = {&b.vmid, &b.dv, &b.G, &b.dS, &b.Gv, &b.r, &b.rp, &b.Gp,
                          &b.vbest, &b.v1, &b.v0, &b.vin, &b.dotv, &b.xi};
         for (double **p : d2)
@@ -1234,20 +1238,21 @@ int co_ensure_capacity(co_ctx *c, int N, int m) {
         b.cap = cap;
         // set 1 is allocated with set 0, never on first use: the Picard maps
         // that use it are captured into CUDA graphs, where no allocation may run
-        if ((rc = ensure_gs(c))) return rc;
+        if ((rc = ensure_gs(c))) {
+            b.cap = 0;
+            return rc;
+        }
         double **lazy[] = {&b.Gk, &b.Phi, &b.Adef, &b.aa, &b.pc};  // re-created at the new size on use
         for (double **q : lazy) {
             if (*q) cudaFree(*q);
             *q = nullptr;
         }
         b.aa_m = 0;
-        if (b.m_cap > 0) {
-            if ((rc = grow(&b.dF, n2 * b.m_cap))) return rc;
-            if ((rc = grow(&b.dG, n2 * b.m_cap))) return rc;
-        }
+        if (m < m_cap) m = m_cap;
     }
     if (m > b.m_cap) {
         size_t n2 = 2 * (size_t)b.cap;
+        b.m_cap = 0;
         if ((rc = grow(&b.dF, n2 * m))) return rc;
         if ((rc = grow(&b.dG, n2 * m))) return rc;
         b.m_cap = m;

@@ -50,7 +50,7 @@ void co_step_free(co_ctx *c) {
 static int step_ensure(co_ctx *c, int N) {
     if (!c->sb) {
         c->sb = (co_step_bufs *)calloc(1, sizeof(co_step_bufs));
-        if (!c->sb) return CO_ERR_NOMEM;
+        if (!c->sb) return co_nomem();
     }
     co_step_bufs *s = c->sb;
     if (N <= s->cap && s->red) return CO_OK;
@@ -67,7 +67,7 @@ static int step_ensure(co_ctx *c, int N) {
         cudaMalloc(&s->keep, n2) != cudaSuccess || cudaMalloc(&s->hv, n2) != cudaSuccess ||
         cudaMalloc(&s->hw, sizeof(double) * (size_t)cap) != cudaSuccess ||
         cudaMalloc(&s->red, sizeof(double) * (CO_STEP_RED + 1)) != cudaSuccess)
-        return CO_ERR_NOMEM;
+        return co_nomem();
     s->cap = cap;
     return CO_OK;
 }
