@@ -799,10 +799,21 @@ static co_dev_opts dev_opts(const co_opts *o, double floor_extra) {
     return d;
 }
 
+// Whether a solve on fixed-point pair sums should end here: the operands' range left them
+// to FP64 arithmetic, or the residual's best so far is behind the pace of FIXED_PACE
+// iterations to the tolerance, in decades (from the sixth on; the first five tell little).
+#define FIXED_PACE 80
+static bool fixed_hopeless(const co_solver_state *st, const co_dev_opts &d) {
+    if (st->wide) return true;
+    const double goal = fmax(d.tol * st->nrm_v, d.abs_floor);
+    return st->k >= 6 && log(st->nrm_r0 / st->nrm_best) * FIXED_PACE < st->k * log(st->nrm_r0 / goal);
+}
+
 // The Anderson loop on device buffers mb.v1 (in/out), mb.v0, mb.w.
-// precision selects the pair kernel of the maps.
+// precision selects the pair kernel of the maps. attempt: the caller starts again where
+// this does not converge, so it ends without a result (done = 0) as soon as it is hopeless.
 static int anderson_loop(co_ctx *c, const co_opts *o, int precision, int N, double S0, double dt,
-                         co_dev_opts d, int max_iter, int *iters_out) {
+                         co_dev_opts d, int max_iter, int *iters_out, bool attempt = false) {
     int rc;
     co_bufs &b = c->mb;
     int n2 = 2 * N;
@@ -838,6 +849,7 @@ static int anderson_loop(co_ctx *c, const co_opts *o, int precision, int N, doub
                     c->st_host->done == 1 ? "  [converged]"
                     : c->st_host->done == 2 ? "  [stagnated]" : "");
         if (c->st_host->done) break;
+        if (attempt && (k == max_iter || fixed_hopeless(c->st_host, d))) return CO_OK;
     }
     if (k > max_iter) {
         k_set_done<<<1, 32, 0, c->stream>>>(c->st, 3);
@@ -855,10 +867,15 @@ static int anderson_loop(co_ctx *c, const co_opts *o, int precision, int N, doub
 }
 
 // Iterations that step_anderson! gives the fixed-point pair sums before it starts again
-// in FP64. 245 of 260 steps of 10,000 markers converge within 48, in 10 to 46 iterations,
-// 1.7e-12 and less from the FP64 solve (11 iterations: 28.9 -> 5.8 ms); the others, which
-// cannot be told by their residuals earlier, pay 20 to 24 ms for the attempt, on 130 to 430.
+// in FP64, and the fewest it is worth starting for. An iteration of an attempt costs 0.2
+// of an FP64 one (0.3 at 390 markers). 374 steps of 600 to 40,000 markers, on two meshes,
+// with dt from 0.001 to 0.02: 293 converge in their attempt, most in 10 to 20 iterations,
+// 5e-12 and less from the FP64 solve; the other 81 give its bits and take 2 % longer on
+// average, 13 % at most (without FIXED_PACE 55 start again, and take 12 % longer); all
+// together 67.7 -> 54.8 s. No rule on the residual tells the two kinds apart much better:
+// some that converge in 40 iterations stall for 30.
 #define FIXED_ITERS 48
+#define FIXED_MIN_ITERS 8
 
 // step_anderson! on device buffers: mb.v1 (guess in, solution out), mb.v0, mb.w
 int co_step_anderson_buffers(co_ctx *c, const co_opts *o, int N, double S0, double dt,
@@ -897,7 +914,8 @@ int co_step_anderson_buffers(co_ctx *c, const co_opts *o, int N, double S0, doub
     }
     co_dev_opts d = dev_opts(o, 0.0);
     int solved = 0;
-    if (o->model == CO_MODEL_LANDAU) {
+    if (o->model == CO_MODEL_LANDAU && o->max_iter >= FIXED_MIN_ITERS &&
+        (o->tol > 0.0 || o->abs_floor > 0.0)) {
         // most solves converge before the iteration has multiplied the last bits of the
         // pair sums into the result; the others start again below, in FP64
         co_fixed_scope fx(c);
@@ -905,8 +923,10 @@ int co_step_anderson_buffers(co_ctx *c, const co_opts *o, int N, double S0, doub
             const size_t bytes = 2 * (size_t)N * sizeof(double);
             CO_CK(cudaMemcpyAsync(c->mb.vin, c->mb.v1, bytes, cudaMemcpyDeviceToDevice, c->stream));
             const int cap = o->max_iter < FIXED_ITERS ? o->max_iter : FIXED_ITERS;
-            if ((rc = anderson_loop(c, o, CO_PREC_FP64, N, S0, dt, d, cap, &it))) return rc;
-            solved = c->st_host->done == 1;
+            rc = anderson_loop(c, o, CO_PREC_FP64, N, S0, dt, d, cap, &it, true);
+            // a residual that is not finite is for the FP64 solve to report
+            if (rc && rc != CO_ERR_NONFINITE) return rc;
+            solved = !rc && c->st_host->done == 1;
             if (!solved)
                 CO_CK(cudaMemcpyAsync(c->mb.v1, c->mb.vin, bytes, cudaMemcpyDeviceToDevice,
                                       c->stream));
