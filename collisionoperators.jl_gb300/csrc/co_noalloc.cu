@@ -35,11 +35,11 @@
 #include <mutex>
 
 #include "co_internal.cuh"
+#include "co_pair64.cuh"
 
 #define CO_NOALLOC_MAX_N 32768
 #define CO_NOALLOC_SLICES 8
 #define NA_TPB 128
-#define NA_R2_MIN_BITS 0x3B282DB34012B251LL  // bit pattern of 1e-24
 
 // 8 slices x 2 components x 32768 markers of FP64 = 4 MiB per device, then a
 // 256-byte tail whose first word is the non-finite flag of the current call
@@ -112,7 +112,7 @@ k_noalloc_pair(const double *__restrict__ v, const double *__restrict__ w,
             double d2 = xg2 - sx2[k];
             double r2 = d1 * d1;
             r2 = fma(d2, d2, r2);
-            bool ok = __double_as_longlong(r2) >= NA_R2_MIN_BITS;
+            bool ok = __double_as_longlong(r2) >= CO_R2_MIN_BITS;
             double y = na_rsqrt(ok ? r2 : 1.0);
             double g1 = sg1[k] - Gg1;
             double g2 = sg2[k] - Gg2;

@@ -4,7 +4,7 @@
 #pragma once
 
 // bit pattern of 1e-24 (functions.jl:224 guard)
-#define CO_R2_MIN_BITS 0x3B282DB34012B251LL
+#define CO_R2_MIN_BITS 0x3AF357C299A88EA7LL
 
 __device__ __forceinline__ double rsqrt_seed64(double x) {
     // FP32 value of x from its high word (x in [1e-30, 1e30], positive)
