@@ -247,7 +247,9 @@ k_mlp_train(const __nv_bfloat16 *__restrict__ wbf, const float *__restrict__ mas
 #pragma unroll
         for (int c = 0; c < 4; c++) gW1[r][c] = gW2[r][c] = 0.f;
     double loss = 0.0;
-    for (int s0 = blockIdx.x * MLP_T; s0 < B; s0 += gridDim.x * MLP_T) {
+    const int tiles = (B - 1) / MLP_T + 1;   // counted in tiles: a sample index would overflow
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int s0 = tile * MLP_T;
         __syncthreads();
         load_inputs(X, n_in, s0, B, nullptr, sm.x);
         load_weights(wbf + o.W0, MLP_H, n_in, true, sm.w);
