@@ -965,13 +965,19 @@ static int ensure_gs(co_ctx *c) {
     return CO_OK;
 }
 
-// Markers of a sort chunk (one block of the locate and placement kernels). Up to
-// 16,384 markers chunks of 256: four times the blocks, and 8 instead of 32 warp turns
-// in the placement; the per-chunk histograms stay at 64 rows, which k_cellcount walks
-// in order, so larger sets keep 1,024. The sorted order does not depend on it.
-static int sort_chunk(int N) { return N <= 64 * 256 ? 256 : CO_CHUNK; }
+// Markers of a sort chunk (one block of the locate and placement kernels): 256 give four
+// times the blocks of 1,024 and 8 instead of 32 warp turns in the placement, against a
+// histogram row per chunk that k_cellcount walks in order. Projection with 256 and with
+// 1,024 on 32 x 32 elements: 59 and 63 us at 2,048 markers, 88 and 99 at 16,384, 90 and 101
+// at 20,000, 109 and 114 at 32,768, 117 and 117 at 49,152, 132 and 130 at 65,536 (16 x 16
+// and 64 x 64 alike); the line lies between the last gain and the first loss. The sorted
+// order does not depend on it.
+#define SMALL_CHUNK 256
+#define SMALL_CHUNK_N (160 * SMALL_CHUNK)
+static int sort_chunk(int N) { return N <= SMALL_CHUNK_N ? SMALL_CHUNK : CO_CHUNK; }
 static size_t sort_rows(int cap) {   // histogram rows for any N <= cap
-    const int a = co_cdiv(cap, CO_CHUNK), b = co_cdiv(cap < 64 * 256 ? cap : 64 * 256, 256);
+    const int a = co_cdiv(cap, CO_CHUNK);
+    const int b = co_cdiv(cap < SMALL_CHUNK_N ? cap : SMALL_CHUNK_N, SMALL_CHUNK);
     return a > b ? a : b;
 }
 
