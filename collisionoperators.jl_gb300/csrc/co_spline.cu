@@ -444,8 +444,8 @@ k_mass2(const double *__restrict__ Minv2, const double *__restrict__ y0,
 // Gauss point plus the logarithm. One thread per Gauss point takes f and the
 // logarithm (most of the work, and a long latency), one per row the sums over it, in
 // the order of q2: with one thread per row for both, the six logarithms of a row
-// followed each other and the smallest meshes ran on a dozen blocks. 256 / nq^2
-// elements per block. Fixed summation order: deterministic. Two jobs may share a
+// followed each other and the smallest meshes ran on a dozen blocks. Up to 256 / nq^2
+// elements per block (elem_per_block). Fixed summation order: deterministic. Two jobs may share a
 // launch (blockIdx.y selects), e.g. r at v_mid and S at v_in.
 struct co_elem_job {
     const double *fc;   // spline coefficients (n_dofs)
@@ -454,9 +454,24 @@ struct co_elem_job {
 };
 
 #define ELEM_THREADS 256
-static int elem_per_block(int nq) { return ELEM_THREADS / (nq * nq); }
+// Elements of a block, up to one point per thread: the count that leaves the busiest SM the
+// least to do, a block counting as two elements more for its barriers (with one or two
+// elements a block, 96 x 96 elements took 132 us a call instead of 72), the larger of
+// equals. With seven always (six points a row), 48 x 48 elements made 330 blocks, three on
+// some of 152 SMs: entropy 46 us a call, 39 with four.
+static int elem_per_block(const co_ctx *c, int jobs) {
+    int best = 0, least = 0;
+    for (int e = ELEM_THREADS / (c->nq * c->nq); e > 0; e--) {
+        const int load = co_cdiv((long long)jobs * co_cdiv(c->n_el, e), c->nsm) * (e + 2);
+        if (best == 0 || load < least) {
+            best = e;
+            least = load;
+        }
+    }
+    return best;
+}
 __global__ void __launch_bounds__(ELEM_THREADS)
-k_elem(co_elem_job j0, co_elem_job j1, int n1, int n2, int nd1, int nq,
+k_elem(co_elem_job j0, co_elem_job j1, int n1, int n2, int nd1, int nq, int epb,
        const double *__restrict__ Tq1, const double *__restrict__ Tq2,
        const double *__restrict__ qw, const double *__restrict__ bp1,
        const double *__restrict__ bp2, int logsq) {
@@ -465,7 +480,7 @@ k_elem(co_elem_job j0, co_elem_job j1, int n1, int n2, int nd1, int nq,
     __shared__ double val[ELEM_THREADS];        // integrand (mode 0) or f log f of a point
     const co_elem_job jb = blockIdx.y ? j1 : j0;
     const int mode = jb.mode, np = nq * nq;
-    const int epb = ELEM_THREADS / np, n_el = n1 * n2;
+    const int n_el = n1 * n2;
     const int t = threadIdx.x;
     // row view: element el, row q1
     const int el = t / nq, q1 = t - el * nq, e = blockIdx.x * epb + el;
@@ -1074,8 +1089,9 @@ int co_project_sorted(co_ctx *c, double *f_out) { return co_project_two(c, f_out
 int co_r_and_entropy_dev(co_ctx *c, const double *f, double *r, const double *fS) {
     co_elem_job jr = {f, 0, c->E};
     co_elem_job js = {fS, 1, c->Ep};
-    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), fS ? 2 : 1), ELEM_THREADS,
-              0, jr, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
+    const int epb = elem_per_block(c, fS ? 2 : 1);
+    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, epb), fS ? 2 : 1), ELEM_THREADS, 0, jr, js, c->n1,
+              c->n2, c->nd1, c->nq, epb, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
               (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     k_dofgather<<<dim3(co_cdiv(c->n_dofs, 128), 1), 128, 0, c->stream>>>(
         c->E, r, c->E, r, c->n1, c->n2, c->nd1, c->nd2);
@@ -1087,8 +1103,9 @@ int co_r_and_entropy_dev(co_ctx *c, const double *f, double *r, const double *fS
 int co_r_solve_dev(co_ctx *c, const double *f, double *L, const double *fS) {
     co_elem_job jr = {f, 0, c->E};
     co_elem_job js = {fS, 1, c->Ep};
-    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), fS ? 2 : 1), ELEM_THREADS,
-              0, jr, js, c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
+    const int epb = elem_per_block(c, fS ? 2 : 1);
+    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, epb), fS ? 2 : 1), ELEM_THREADS, 0, jr, js, c->n1,
+              c->n2, c->nd1, c->nq, epb, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
               (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     c->launches++;
     CO_CK(cudaGetLastError());
@@ -1101,8 +1118,9 @@ int co_compute_r_dev(co_ctx *c, const double *f, double *r) {
 
 int co_entropy_parts_dev(co_ctx *c, const double *f) {
     co_elem_job js = {f, 1, c->Ep};
-    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, elem_per_block(c->nq)), 1), ELEM_THREADS, 0, js, js,
-              c->n1, c->n2, c->nd1, c->nq, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
+    const int epb = elem_per_block(c, 1);
+    co_launch(c, k_elem, dim3(co_cdiv(c->n_el, epb), 1), ELEM_THREADS, 0, js, js, c->n1, c->n2,
+              c->nd1, c->nq, epb, c->Tq1, c->Tq2, c->qw, c->bp1, c->bp2,
               (c->flags & CO_FLAG_LOGSQ) ? 1 : 0);
     c->launches++;
     CO_CK(cudaGetLastError());
