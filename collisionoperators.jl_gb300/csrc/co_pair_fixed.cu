@@ -31,11 +31,13 @@
 // is 2^-8 of the scale. A pair with |d| below 2^-9 of the scaled domain or |g| below
 // 2^-9 of the largest G is taken from all three words, g shifted left like d
 // (fx_refine), so that its error is relative to its own |d| and |g|: less than one pair
-// in a hundred in the distributions of the performance cases. Where the bounds of 32
-// targets and 32 sources rule such pairs out (80 % of the group pairs at 131,072 markers,
-// 2 to 20 % where G has strong outliers), a loop without the test and the FP64 form runs.
-// 131,072 markers: 58.0 ms, 58.7 with two words for every pair, 62.3 with the test in
-// every loop, 67.2 with three words for every pair.
+// in a hundred in the distributions of the performance cases. The bounds of 32 targets and
+// 32 sources pick one of three loops: neither can be small (80 % of the group pairs for a
+// smooth G, 2 to 20 % where the largest G is 25 to 40 times the median), only |g| can, or
+// |d| can, the only one with the FP64 form. 131,072 markers: 57.9 ms; 58.7 with two words
+// for every pair, 62.3 with the test in every loop, 67.2 with three words for every pair.
+// A map of 16,384 markers with strong outliers in G: 1.13 ms with two words for every pair,
+// 1.19 with one loop for both kinds of small pairs, 1.17 now.
 //
 // Close pairs: |d| < 2^-22 of the scaled domain (a few 1e-6 for [-6, 6]^2) take
 // the FP64 form from the FP64 operands, including the |d|^2 < 1e-24 guard of
@@ -145,19 +147,19 @@ __device__ __forceinline__ void fixed_terms(fx64 S, const fx_limb &y3, fx_limb w
     }
 }
 
-// Whether any of 32 targets and 32 sources may differ by little in x or in G, from the
-// bounds of the high words (their difference is that of the values, or one less)
-__device__ __forceinline__ bool fixed_near(const co_fixed_ops &o, int gt, int gs) {
+// Whether any of 32 targets and 32 sources may differ by little, from the bounds of the high
+// words (their difference is that of the values, or one less): 2 in x, 1 in G alone, 0 no
+__device__ __forceinline__ int fixed_near(const co_fixed_ops &o, int gt, int gs) {
     const int4 l = o.box[2 * gt], h = o.box[2 * gt + 1], sl = o.box[2 * gs], sh = o.box[2 * gs + 1];
     const int x = max(max(sl.x - h.x, l.x - sh.x), max(sl.y - h.y, l.y - sh.y));
     const int g = max(max(sl.z - h.z, l.z - sh.z), max(sl.w - h.w, l.w - sh.w));
-    return x < o.x_near || g < (1 << FX_SMALL_G);
+    return x < o.x_near ? 2 : g < (1 << FX_SMALL_G);
 }
 
 // 32 rotation steps: this warp's 32 targets against the 32 sources of group grp of
-// tile J; SRC: the sources' sums too; NEAR: small differences among them. Signs are
-// applied when the sums are written.
-template <int W, int NC, bool SRC, bool UNI, bool NEAR>
+// tile J; SRC: the sources' sums too; NEAR: small differences among them (fixed_near).
+// Signs are applied when the sums are written.
+template <int W, int NC, bool SRC, bool UNI, int NEAR>
 __device__ __forceinline__ void fixed_group(fixed_smem<W, NC> &sm, const co_fixed_ops &o,
                                             const fixed_target &t, int ig, int J, int grp,
                                             int lane, const double (&tf)[2], fx_acc (&a)[NC],
@@ -174,9 +176,9 @@ __device__ __forceinline__ void fixed_group(fixed_smem<W, NC> &sm, const co_fixe
         const fx_limb k1 = {ga.x - t.g.x, ga.y - t.g.y}, k2 = {t.g.z - ga.z, t.g.w - ga.w};
         fx_fine p = fx_plain(xa.x - t.x.x, xa.y - t.x.y, k1, k2);
         bool close = false;
-        if (NEAR && (p.d.m < o.m_small || fx_within(k1.h, k2.h, FX_SMALL_G))) {
+        if (NEAR && ((NEAR == 2 && p.d.m < o.m_small) || fx_within(k1.h, k2.h, FX_SMALL_G))) {
             const int ia = J * TS + j;
-            close = p.d.m < o.m_close;
+            close = NEAR == 2 && p.d.m < o.m_close;
             if (close) {
                 const close_term c = pair_close64(o.px[ig], o.pg[ig], o.px[ia], o.pg[ia]);
                 const double uf = o.unit[0], ua = o.unit[2];   // into scaled units
@@ -194,7 +196,7 @@ __device__ __forceinline__ void fixed_group(fixed_smem<W, NC> &sm, const co_fixe
         }
         // the source's sum passes on: lane - 1 may add to it in the next step, and the
         // shuffles below do not order shared memory between lanes
-        if (SRC && NEAR) __syncwarp();
+        if (SRC && NEAR == 2) __syncwarp();
         const fx_limb y3 = fx_invcube(p.d.c1, p.d.c2);
         const fx64 S = fx_mul(fx_split(fx_cross(p.k1, p.k2, p.d.c1, p.d.c2)), y3);
         fx64 T[NC], U[NC];
@@ -268,15 +270,19 @@ __device__ __forceinline__ void fixed_item(fixed_smem<W, NC> &sm, const co_fixed
         for (int rr = 0; rr < W; rr++) {
             const int grp = (warp + rr) & (W - 1);
             if (k == 0) {
-                if (uni) fixed_group<W, NC, false, true, true>(sm, o, t, ig, J, grp, lane, tf, a, gd);
-                else fixed_group<W, NC, false, false, true>(sm, o, t, ig, J, grp, lane, tf, a, gd);
+                if (uni) fixed_group<W, NC, false, true, 2>(sm, o, t, ig, J, grp, lane, tf, a, gd);
+                else fixed_group<W, NC, false, false, 2>(sm, o, t, ig, J, grp, lane, tf, a, gd);
             } else {
-                if (fixed_near(o, I * W + warp, J * W + grp)) {
-                    if (uni) fixed_group<W, NC, true, true, true>(sm, o, t, ig, J, grp, lane, tf, a, gd);
-                    else fixed_group<W, NC, true, false, true>(sm, o, t, ig, J, grp, lane, tf, a, gd);
+                const int near = fixed_near(o, I * W + warp, J * W + grp);
+                if (near == 2) {
+                    if (uni) fixed_group<W, NC, true, true, 2>(sm, o, t, ig, J, grp, lane, tf, a, gd);
+                    else fixed_group<W, NC, true, false, 2>(sm, o, t, ig, J, grp, lane, tf, a, gd);
+                } else if (near) {
+                    if (uni) fixed_group<W, NC, true, true, 1>(sm, o, t, ig, J, grp, lane, tf, a, gd);
+                    else fixed_group<W, NC, true, false, 1>(sm, o, t, ig, J, grp, lane, tf, a, gd);
                 } else {
-                    if (uni) fixed_group<W, NC, true, true, false>(sm, o, t, ig, J, grp, lane, tf, a, gd);
-                    else fixed_group<W, NC, true, false, false>(sm, o, t, ig, J, grp, lane, tf, a, gd);
+                    if (uni) fixed_group<W, NC, true, true, 0>(sm, o, t, ig, J, grp, lane, tf, a, gd);
+                    else fixed_group<W, NC, true, false, 0>(sm, o, t, ig, J, grp, lane, tf, a, gd);
                 }
                 __syncthreads();
             }
