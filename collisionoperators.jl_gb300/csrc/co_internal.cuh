@@ -156,6 +156,7 @@ struct co_ctx {
     int pair_split_fp64, pair_split_fp32;  // split factors of the plain kernels (0 = auto)
     int pair_symmetric;      // 1: Newton's-third-law kernels (default), 0: one-sided
     int nsm;
+    int elem_block[2];         // elements per block of the quadrature, for one and two jobs
     int early;                 // co_launch: grids start before the one before them ends
     int fixed_ex;            // exponent of the fixed-point pair sum's coordinate scale
     // launch counter (kernels of this library launched through the context)

@@ -387,7 +387,7 @@ __device__ __forceinline__ int scale_exp(double x) {
 // times the others: 2^-2 to 2^-5.5 and 0.1 to 0.7 times FP64's error for k = 0 to 5, 2^-6.4
 // and 1.2 times for k = 6). Thermal distributions with the solver's own G: 2^-4 and more.
 // Markers so close together in their domain that most pairs would be close ones are left
-// to the FP64 loop too (half-width 1e6 for thermal width 1). 2 us of a map of 2,048 markers.
+// to the FP64 loop too (half-width 1e6 for thermal width 1).
 #define FIXED_SAMPLES 64
 __device__ __forceinline__ bool fixed_wide(const float4 *sv, const float *swt, float x1, float x2,
                                            float G1, float G2, bool force) {
@@ -400,8 +400,7 @@ __device__ __forceinline__ bool fixed_wide(const float4 *sv, const float *swt, f
         const float r2 = fmaf(d2, d2, d1 * d1);
         near += r2 < 0x1p-40f;
         const float r = r2 > 0.f ? fminf(rsqrt_normal(r2), 64.f) : 0.f;   // 0: the marker itself
-        const float gg = fmaf(g2, g2, fmaf(g1, g1, 0x1p-80f));
-        const float q = gg * rsqrt_normal(gg) * r;
+        const float q = fmaxf(fabsf(g1), fabsf(g2)) * r;
         num = fmaf(swt[s], q, num);
         gr += q;
         wr = fmaf(swt[s], r, wr);
@@ -423,7 +422,11 @@ __device__ __forceinline__ fx64 fx_round(double a, int &rest) {
 // (max is order-free), so the scales are one set for the launch. A non-finite operand (maximum inf) makes every
 // vdot NaN, as the FP64 sum does. unit[0], unit[2]: FP64 terms of F and A into
 // scaled units; unit[1], unit[3]: scaled sums back to vdot and A.
-__global__ void __launch_bounds__(256)
+// Threads: the 60 FP64 operations and conversions of a marker queue on its SM's FP64 pipe, so
+// blocks are small: at 2,048 markers 11.2 us with 256 threads, 7.7 with 64 (ncu, cold).
+#define FIXED_PACK 64
+static_assert(FIXED_PACK == FIXED_SAMPLES, "a sample per thread");
+__global__ void __launch_bounds__(FIXED_PACK)
 k_pair_fixed_pack(const double2 *__restrict__ px, const double2 *__restrict__ pg,
                   const double *__restrict__ pw, const int *__restrict__ Mp,
                   const double2 *__restrict__ part, int npart, int ex, double c1, double c2,
@@ -431,10 +434,24 @@ k_pair_fixed_pack(const double2 *__restrict__ px, const double2 *__restrict__ pg
                   int4 *__restrict__ box, fx64 *__restrict__ ow, double *__restrict__ pwn,
                   double *__restrict__ unit, int *__restrict__ wide) {
     co_grid_wait();
-    __shared__ double shg[8], shw[8];
+    __shared__ double shg[FIXED_PACK / 32], shw[FIXED_PACK / 32];
     __shared__ float4 sv[FIXED_SAMPLES];   // x1 x2 g1 g2, scaled
     __shared__ float swt[FIXED_SAMPLES];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // all loads first: their latency passes with that of the maxima
+    const int M = *Mp;
+    const int p = blockIdx.x * blockDim.x + tid;   // below Mpad: the blocks are whole
+    const double2 zero = make_double2(0.0, 0.0);
+    const double2 x = p < M ? px[p] : zero, G = p < M ? pg[p] : zero;
+    const double w = p < M ? pw[p] : 0.0;
+    double2 xs = zero, Gs = zero;
+    double ws = 0.0;
+    if (M > 0) {
+        const int q = (int)((long long)tid * M / FIXED_SAMPLES);
+        xs = px[q];
+        Gs = pg[q];
+        ws = pw[q];
+    }
     double gm = 0.0, wm = 0.0;
     for (int i = tid; i < npart; i += blockDim.x) {
         const double2 q = part[i];
@@ -450,7 +467,7 @@ k_pair_fixed_pack(const double2 *__restrict__ px, const double2 *__restrict__ pg
         shw[warp] = wm;
     }
     __syncthreads();
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < FIXED_PACK / 32; i++) {
         gm = fmax(gm, shg[i]);
         wm = fmax(wm, shw[i]);
     }
@@ -463,24 +480,17 @@ k_pair_fixed_pack(const double2 *__restrict__ px, const double2 *__restrict__ pg
         unit[2] = ldexp(1.0, ex);
         unit[3] = ok ? ldexp(1.0, ew - ex) : nan("");
     }
-    const int M = *Mp;
-    if (tid < FIXED_SAMPLES && M > 0) {
-        const int q = (int)((long long)tid * M / FIXED_SAMPLES);
-        const double2 x = px[q], G = pg[q];
-        sv[tid] = make_float4((float)((x.x - c1) * sx), (float)((x.y - c2) * sx), (float)(G.x * sg),
-                              (float)(G.y * sg));
-        swt[tid] = (float)fabs(pw[q] * sw);
-    }
-    const int p = blockIdx.x * blockDim.x + tid;   // below Mpad: the blocks are whole
+    sv[tid] = make_float4((float)((xs.x - c1) * sx), (float)((xs.y - c2) * sx), (float)(Gs.x * sg),
+                          (float)(Gs.y * sg));
+    swt[tid] = (float)fabs(ws * sw);
     // padding: outside the scaled domain (coordinates stay below 1/2), weight 0
     double x1 = 0.96875, x2 = 0.96875, G1 = 0.0, G2 = 0.0, wn = 0.0;
     if (p < M) {
-        const double2 x = px[p], G = pg[p];
         x1 = (x.x - c1) * sx;
         x2 = (x.y - c2) * sx;
         G1 = G.x * sg;
         G2 = G.y * sg;
-        wn = pw[p] * sw;
+        wn = w * sw;
     }
     int4 r;
     const fx64 V1 = fx_round(G1 * 0x1p60, r.z), V2 = fx_round(G2 * 0x1p60, r.w);
@@ -523,7 +533,7 @@ int co_pair_fixed_pack(co_ctx *c, int Mub, int npart) {
     const int ex = ilogb(big) + 2;
     c->fixed_ex = ex;
     const int Mpad = co_cdiv(Mub, 256) * 256;
-    co_launch(c, k_pair_fixed_pack, Mpad / 256, 256, 0, b.px, b.pg, b.pw, b.cstart + c->n_el,
+    co_launch(c, k_pair_fixed_pack, Mpad / FIXED_PACK, FIXED_PACK, 0, b.px, b.pg, b.pw, b.cstart + c->n_el,
               b.gwmax, npart, ex, c1, c2, (longlong2 *)b.fx_x, b.fx_g, b.fx_rest,
               b.fx_box, b.fx_w, b.pwn, b.unit, &c->st->wide);
     c->launches++;

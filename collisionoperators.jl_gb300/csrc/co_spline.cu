@@ -459,7 +459,7 @@ struct co_elem_job {
 // elements a block, 96 x 96 elements took 132 us a call instead of 72), the larger of
 // equals. With seven always (six points a row), 48 x 48 elements made 330 blocks, three on
 // some of 152 SMs: entropy 46 us a call, 39 with four.
-static int elem_per_block(const co_ctx *c, int jobs) {
+static int elem_per_block_of(const co_ctx *c, int jobs) {
     int best = 0, least = 0;
     for (int e = ELEM_THREADS / (c->nq * c->nq); e > 0; e--) {
         const int load = co_cdiv((long long)jobs * co_cdiv(c->n_el, e), c->nsm) * (e + 2);
@@ -470,6 +470,7 @@ static int elem_per_block(const co_ctx *c, int jobs) {
     }
     return best;
 }
+static int elem_per_block(const co_ctx *c, int jobs) { return c->elem_block[jobs - 1]; }
 __global__ void __launch_bounds__(ELEM_THREADS)
 k_elem(co_elem_job j0, co_elem_job j1, int n1, int n2, int nd1, int nq, int epb,
        const double *__restrict__ Tq1, const double *__restrict__ Tq2,
@@ -1195,6 +1196,7 @@ int co_loggrad_dev(co_ctx *c, const double *x, int N, const double *f, double *g
 
 // dynamic shared memory of the sort kernels (one int per cell)
 int co_spline_configure(co_ctx *c) {
+    for (int jobs = 1; jobs <= 2; jobs++) c->elem_block[jobs - 1] = elem_per_block_of(c, jobs);
     int bytes = (int)(sizeof(int) * (size_t)c->n_el);
     if (bytes > 48 * 1024) {
         if (bytes > 200 * 1024) return CO_ERR_UNSUPPORTED;
