@@ -287,7 +287,8 @@ static inline int co_pack_mode(int precision) {
 }
 // Whether an FP64-accurate pair sum of up to Mub markers takes the fixed-point
 // kernel: from four 128-marker tiles on; below that the one-sided FP64 kernel's
-// single launch is as fast. The one-sided FP64 form also stays for CO_FLAG_ONESIDED.
+// single launch is as fast. The one-sided FP64 form also stays for CO_FLAG_ONESIDED, and
+// operands whose range is too wide take FP64 arithmetic inside the kernel (fixed_wide).
 // Calls that evaluate the sum once take it (co_fixed_scope). A solve repeats it, and on a
 // stiff map the iteration multiplies a difference of 1e-16 until the solve stops at
 // another iterate (3 of 40 steps of 10,000 markers, 3 of 14 batches, by 1e-6 to 1e-4):

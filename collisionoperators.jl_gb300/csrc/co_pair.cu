@@ -7,9 +7,11 @@
 // into slices whose partial sums are added afterwards in slice order, so
 // results are bitwise reproducible for a given N.
 //
-// The reference's Float64 path runs on the fixed-point kernels of co_pair_fixed.cu;
-// the FP64 arithmetic below serves the one-sided kernels (CO_FLAG_ONESIDED, fewer
-// than 385 markers) and the batch engine. On GB300 FP64 issues at 1/64 of the FP32
+// Calls that evaluate the Float64 sum once run on the fixed-point kernels of
+// co_pair_fixed.cu, as do the first iterations of step_anderson!. The FP64 arithmetic
+// below (its symmetric loop in co_pair64.cuh) serves the solves, the predictor, the batch
+// engine, the one-sided kernels (CO_FLAG_ONESIDED, fewer than 385 markers) and operands
+// whose range is too wide for fixed point. On GB300 FP64 issues at 1/64 of the FP32
 // rate, so the per-pair FP64 instruction count is what sets its time. The pair body
 // is 20 FP64 instructions:
 //   d (2), |d|^2 (2), 1/|d| refinement (5), G difference (2), d.g (2),
@@ -1223,7 +1225,7 @@ int co_ensure_part(co_ctx *c, size_t n) {
 
 #define SYM_KC 8
 
-// FP64 symmetric pair sum on the padded operands (batch instances)
+// FP64 symmetric pair sum on the padded operands (solves and predictors)
 static int pair64_sym(co_ctx *c, int Mub) {
     const int nt = co_cdiv(Mub, ST), H = nt / 2, KC = SYM_KC, nchunk = co_cdiv(H + 1, KC);
     const size_t gsz = (size_t)nchunk * nt * 2 * ST, asz = (size_t)(H > 0 ? H : 1) * nt * 2 * ST;

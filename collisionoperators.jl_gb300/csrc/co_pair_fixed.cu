@@ -5,13 +5,14 @@
 // take 10 clocks of an SM per lane. 32 x 32 -> 64-bit multiply-adds run at 64
 // lanes per clock, beside 128 lanes of 32-bit adds, so the pair term is evaluated
 // in 64-bit fixed point (co_pair_fixed.cuh): 34 wide multiply-adds, which issue at
-// about 32 lanes per clock where they have distinct operands, and some 130 adds,
-// shifts and moves. What bounds it is that multiply pipe (73 % busy) with the issue
-// slots (60 %): 2.0 clocks per pair and SM lane. At 131,072 markers (8.6e9 pairs) the
+// about 32 lanes per clock where they have distinct operands, and some 140 adds,
+// shifts and moves. What bounds it is that multiply pipe (76 % busy) with the issue
+// slots (64 %): 2.0 clocks per pair and SM lane. At 131,072 markers (8.6e9 pairs) the
 // sum takes 58 ms against 352 for the FP64 kernel it replaces, at 16,384 0.95 against
 // 6.4; F with the metric at 10,000 markers 0.70 against 6.4 (one-sided FP64).
-// Measured error of vdot (2-norm, against 80-bit sums): 1.3e-16 to 2e-16 for 600 to
-// 131,072 markers; the FP64 kernel's is 3.7e-16 to 9.1e-16.
+// Measured error of vdot and of the metric (2-norm, against 80-bit sums): 1.1e-16 to
+// 1.2e-16 for 600 to 10,000 markers, the rounding of the results; the FP64 kernels' is
+// 2.8e-16 to 5.6e-16 for vdot and 2.3e-16 to 4.6e-16 for the metric.
 //
 // Operands (k_pair_fixed_pack). Exact scalings by powers of two bring every
 // coordinate below 1 in units of 2^-61 and every G in units of 2^-60; what that
@@ -24,8 +25,8 @@
 // arithmetic. d is shifted left until it fills its word (float exponent of the
 // larger component); 1/|d|^3 starts from the MUFU seed y of 1/sqrt(r) and takes
 // y^3 (1 - 3e/2 + 15 e^2/8), e = r y^2 - 1, in integers. A term carries an error
-// of about 2e-16 of |g|/|d| (FP64 arithmetic: 2-3e-16), unbiased, and the sums of
-// terms are exact integers, converted to FP64 once per tile pair.
+// of about 1e-16 of |g|/|d| (4e-16 at most; FP64 arithmetic: 2-3e-16), unbiased, and the
+// sums of terms are exact integers, converted to FP64 once per tile pair.
 //
 // Small differences: the rounding of the two-word operands is 2^-53 of a difference that
 // is 2^-8 of the scale. A pair with |d| below 2^-9 of the scaled domain or |g| below

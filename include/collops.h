@@ -100,7 +100,12 @@ int co_ctx_destroy(co_ctx *ctx);
 int co_ctx_n_dofs(const co_ctx *ctx, int *n_dofs);
 
 /* COLLISION_FN: compute_collision! (functions.jl:205-237),
- * compute_collision_gpu! / compute_collision_gpu32! (collision_gpu.jl:233-280). */
+ * compute_collision_gpu! / compute_collision_gpu32! (collision_gpu.jl:233-280).
+ * From 385 markers on, this call, co_collision_metric, co_picard_map (FP64) and
+ * the first iterations of co_step_anderson evaluate the pair sum in 64-bit
+ * fixed point, to a smaller error than FP64 arithmetic; where the coordinates,
+ * G or w span too much for that, the device takes FP64 arithmetic by itself.
+ * CO_FLAG_ONESIDED keeps FP64 arithmetic throughout. */
 int co_collision(co_ctx *ctx, const double *v, const double *w, const double *G,
                  double *dot_v, int N);
 
@@ -139,7 +144,10 @@ int co_picard_map(co_ctx *ctx, const co_opts *opts, double *v_out,
 
 /* step_anderson! (solver.jl:300-423) entirely on the device; v1 is the initial
  * guess in and the solution out. Outputs mirror its return tuple
- * (iterations, residual, n_restarts, initial residual). */
+ * (iterations, residual, n_restarts, initial residual). With CO_PREC_FP64 (Landau)
+ * up to 48 iterations run on the fixed-point pair sums first; where they do not
+ * converge, or cannot, the solve starts again from the guess in FP64 arithmetic,
+ * and the outputs are that solve's. */
 int co_step_anderson(co_ctx *ctx, const co_opts *opts, double *v1,
                      const double *v0, const double *w, int N, double S0,
                      double dt, int *iters, double *res, int *n_restarts,
@@ -416,7 +424,8 @@ int co_ctx_stream(const co_ctx *ctx, void **stream);
 /* Per-kernel timing of the pair sums with CUDA events recorded around each
  * launch on the context's stream. */
 typedef struct {
-    double pair64_ms;                    /* summed event time, FP64 pair kernels */
+    double pair64_ms;                    /* summed event time, FP64 pair kernels
+                                            (fixed-point ones included)          */
     unsigned long long pair64_launches;
     double pair64_pairs;                 /* sum over launches of M (M - 1)      */
     double pair32_ms;                    /* same for the mixed FP32 kernel       */
