@@ -42,7 +42,8 @@
 //
 // Close pairs: |d| < 2^-22 of the scaled domain (a few 1e-6 for [-6, 6]^2) take
 // the FP64 form from the FP64 operands, including the |d|^2 < 1e-24 guard of
-// functions.jl:224; that covers coincident markers.
+// functions.jl:224; that covers coincident markers. So do pairs with |d| below 2^-9 of it
+// where a weight is below 2^-8 of the largest.
 //
 // The metric A = sum_a w_a U(v_g - v_a) of functions.jl:249-290 comes from the same
 // evaluation: U = (d2, -d1) (d2, -d1)^T / |d|^3.
@@ -179,7 +180,9 @@ __device__ __forceinline__ void fixed_group(fixed_smem<W, NC> &sm, const co_fixe
         bool close = false;
         if (NEAR && ((NEAR == 2 && p.d.m < o.m_small) || fx_within(k1.h, k2.h, FX_SMALL_G))) {
             const int ia = J * TS + j;
-            close = NEAR == 2 && p.d.m < o.m_close;
+            // a light weight's product is rounded to 2^-61 of the heaviest over |d|
+            close = NEAR == 2 && (p.d.m < o.m_close ||
+                                  (!UNI && p.d.m < o.m_small && fx_light(sm.w[j], t.w)));
             if (close) {
                 const close_term c = pair_close64(o.px[ig], o.pg[ig], o.px[ia], o.pg[ia]);
                 const double uf = o.unit[0], ua = o.unit[2];   // into scaled units

@@ -163,6 +163,11 @@ FXF fx64 fx_cross(const fx_limb &k1, const fx_limb &k2, const fx_limb &d1, const
 FXF bool fx_within(int32_t a, int32_t b, int n) {
     return (((uint32_t)(a + (1 << n)) | (uint32_t)(b + (1 << n))) >> (n + 1)) == 0;
 }
+// |wa| or |wt| below 2^-8
+FXF bool fx_light(fx64 wa, fx64 wt) {
+    return (uint32_t)(fx_hi(wa) + (1 << 21)) < (1u << 22) ||
+           (uint32_t)(fx_hi(wt) + (1 << 21)) < (1u << 22);
+}
 FXF fx64 fx_join(const fx_limb &a) { return ((fx64)a.h << 31) + a.l; }
 
 // A pair's differences from all 96 bits, K normalised like D, so that the error of its

@@ -98,6 +98,19 @@ def test_cold_core(built_lib, collops_mod, k, share):
     check(collops_mod, graded(6.0), v, w, G)
 
 
+@pytest.mark.parametrize("seed", range(4))
+def test_light_close_pairs(built_lib, collops_mod, seed):
+    """Pairs just beyond the reach of the FP64 form, of markers whose weights lie over eight
+    decades: a light one's term is small, but not its 1/|d|."""
+    v, w, G = _markers(400, 29 + seed)
+    rng = np.random.default_rng(30 + seed)
+    t = rng.uniform(0, 2 * np.pi, 200)
+    gap = 10.0 ** rng.uniform(-5.2, -5, 200)
+    v[200:] = v[:200] + gap[:, None] * np.stack([np.cos(t), np.sin(t)], 1)
+    w *= 10.0 ** (-8 * rng.random(400))
+    check(collops_mod, graded(6.0), v, w, G)
+
+
 def test_tiny_domain(built_lib, collops_mod, oracle_mod):
     """A domain so small that the guard distance 1e-12 is far beyond the usual reach of the
     FP64 form. Against the CPU oracle: sums of N FP64 terms, ten times sqrt(N) 2^-53."""
