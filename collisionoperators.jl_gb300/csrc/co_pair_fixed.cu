@@ -4,7 +4,7 @@
 // GB300 issues FP64 at 1/64 of the FP32 rate: the 20 FP64 instructions of a pair
 // take 10 clocks of an SM per lane. 32 x 32 -> 64-bit multiply-adds run at 64
 // lanes per clock, beside 128 lanes of 32-bit adds, so the pair term is evaluated
-// in 64-bit fixed point (co_pair_fixed.cuh): 34 wide multiply-adds, which issue at
+// in 64-bit fixed point (co_pair_fixed.cuh): 35 wide multiply-adds, which issue at
 // about 32 lanes per clock where they have distinct operands, and some 140 adds,
 // shifts and moves. What bounds it is that multiply pipe (76 % busy) with the issue
 // slots (64 %): 2.0 clocks per pair and SM lane. At 131,072 markers (8.6e9 pairs) the
@@ -25,7 +25,7 @@
 // arithmetic. d is shifted left until it fills its word (float exponent of the
 // larger component); 1/|d|^3 starts from the MUFU seed y of 1/sqrt(r) and takes
 // y^3 (1 - 3e/2 + 15 e^2/8), e = r y^2 - 1, in integers. A term carries an error
-// of about 1e-16 of |g|/|d| (4e-16 at most; FP64 arithmetic: 2-3e-16), unbiased, and the
+// of about 1.2e-16 of |g|/|d| (4e-16 at most; FP64 arithmetic: 2-3e-16), unbiased, and the
 // sums of terms are exact integers, converted to FP64 once per tile pair.
 //
 // Small differences: the rounding of the two-word operands is 2^-53 of a difference that
@@ -36,7 +36,8 @@
 // 32 sources pick one of three loops: neither can be small (80 % of the group pairs for a
 // smooth G, 2 to 20 % where the largest G is 25 to 40 times the median), only |g| can, or
 // |d| can, the only one with the FP64 form. 131,072 markers: 57.9 ms; 58.7 with two words
-// for every pair, 62.3 with the test in every loop, 67.2 with three words for every pair.
+// for every pair, 62.3 with the test in every loop, 67.2 with three words for every pair
+// (59.0 now, with c at y in fx_invcube).
 // A map of 16,384 markers with strong outliers in G: 1.13 ms with two words for every pair,
 // 1.19 with one loop for both kinds of small pairs, 1.17 now.
 //

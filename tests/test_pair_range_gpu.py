@@ -98,6 +98,19 @@ def test_cold_core(built_lib, collops_mod, k, share):
     check(collops_mod, graded(6.0), v, w, G)
 
 
+def test_sums_of_one_term(built_lib, collops_mod):
+    """Each marker 0.005 to 0.02 from one of 32 weighted ones, the others weightless: its sum
+    is next to one term, whose error nothing averages."""
+    v, w, G = _markers(512, 27)
+    rng = np.random.default_rng(28)
+    w = np.where(np.arange(512) % 16 == 0, w, 0.0)
+    t, d = rng.uniform(0, 2 * np.pi, 512), rng.uniform(0.005, 0.02, 512)
+    at = 16 * rng.integers(0, 32, 512)
+    near = v[at] + d[:, None] * np.stack([np.cos(t), np.sin(t)], 1)
+    v = np.where(w[:, None] > 0.0, v, near)
+    check(collops_mod, graded(6.0), v, w, rng.standard_normal((512, 2)))
+
+
 @pytest.mark.parametrize("seed", range(4))
 def test_light_close_pairs(built_lib, collops_mod, seed):
     """Pairs just beyond the reach of the FP64 form, of markers whose weights lie over eight
