@@ -6,10 +6,10 @@
 // lanes per clock, beside 128 lanes of 32-bit adds, so the pair term is evaluated
 // in 64-bit fixed point (co_pair_fixed.cuh): 35 wide multiply-adds, which issue at
 // about 32 lanes per clock where they have distinct operands, and some 140 adds,
-// shifts and moves. What bounds it is that multiply pipe (76 % busy) with the issue
+// shifts and moves. What bounds it is that multiply pipe (78 % busy) with the issue
 // slots (64 %): 2.0 clocks per pair and SM lane. At 131,072 markers (8.6e9 pairs) the
-// sum takes 58 ms against 352 for the FP64 kernel it replaces, at 16,384 0.95 against
-// 6.4; F with the metric at 10,000 markers 0.70 against 6.4 (one-sided FP64).
+// sum takes 59 ms against 352 for the FP64 kernel it replaces, at 16,384 0.97 against
+// 6.4; F with the metric at 10,000 markers 0.71 against 6.4 (one-sided FP64).
 // Measured error of vdot and of the metric (2-norm, against 80-bit sums): 1.1e-16 to
 // 1.2e-16 for 600 to 10,000 markers, the rounding of the results; the FP64 kernels' is
 // 2.8e-16 to 5.6e-16 for vdot and 2.3e-16 to 4.6e-16 for the metric.
@@ -39,7 +39,7 @@
 // for every pair, 62.3 with the test in every loop, 67.2 with three words for every pair
 // (59.0 now, with c at y in fx_invcube).
 // A map of 16,384 markers with strong outliers in G: 1.13 ms with two words for every pair,
-// 1.19 with one loop for both kinds of small pairs, 1.17 now.
+// 1.19 with one loop for both kinds of small pairs, 1.18 now.
 //
 // Close pairs: |d| < 2^-22 of the scaled domain (a few 1e-6 for [-6, 6]^2) take
 // the FP64 form from the FP64 operands, including the |d|^2 < 1e-24 guard of
